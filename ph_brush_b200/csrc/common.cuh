@@ -63,6 +63,10 @@ struct RepDesc {
     long long mesh_off;   // offset (elements) into real / complex mesh arrays
     int oct[3];           // G octant dims (n/2+1)
     long long oct_off;
+    // the same influence kernel unfolded by the stencil's reach on either side, in blocks of
+    // 4 (x) x 8 (y) values (one 128-byte line): entry (x, y, z) holds G at offset (x, y, z) - order
+    int gx_xb, gx_yb;     // blocks per row of blocks, rows of blocks per plane
+    long long gx_off;
     int mod_off[3];       // offsets of the B-spline moduli per axis
     int tw_off[3];        // offsets of the twiddle tables per axis
     int tw_off_h;         // twiddle table of length nx/2 (real-to-complex path)
@@ -158,6 +162,7 @@ struct DevPtrs {
     float2* cmesh;             // complex work mesh
     float* phi;                // potential mesh (real)
     float* goct;               // influence kernel octant
+    float* gext;               // influence kernel with margins, blocked (RepDesc::gx_*)
     float* moduli;
     float2* twiddle;
     float2* thtab;             // per-axis influence factors of the rebuild's z pass

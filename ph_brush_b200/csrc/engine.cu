@@ -599,7 +599,8 @@ static int share_octants(phmc_engine* h) {
     CU(cudaStreamSynchronize(E.stream));
     CU(cudaMemcpy(g.data(), E.d.goct, sizeof(float) * (size_t)E.total_oct, cudaMemcpyDeviceToHost));
     std::map<unsigned long long, std::vector<int>> by_hash;
-    bool changed = false;
+    std::vector<int> own;  // replicas whose octant is the first of its kind
+    long long gx_total = 0;
     for (int r = 0; r < E.R; ++r) {
         RepDesc& D = E.desc[r];
         const size_t n = (size_t)D.oct[0] * D.oct[1] * D.oct[2];
@@ -617,10 +618,21 @@ static int share_octants(phmc_engine* h) {
             if (C.oct[0] == D.oct[0] && C.oct[1] == D.oct[1] && C.oct[2] == D.oct[2] &&
                 std::memcmp(g.data() + C.oct_off, p, n * sizeof(float)) == 0) { same = c; break; }
         }
-        if (same >= 0) { D.oct_off = E.desc[same].oct_off; changed = true; }
-        else seen.push_back(r);
+        // the unfolded table: offsets -order .. n/2 + order per axis (+ 16 in x for whole 4-wide chunks)
+        D.gx_xb = (D.mesh[0] / 2 + 2 * E.order + 1 + 16 + 3) / 4;
+        D.gx_yb = (D.mesh[1] / 2 + 2 * E.order + 1 + 7) / 8;
+        if (same >= 0) { D.oct_off = E.desc[same].oct_off; D.gx_off = E.desc[same].gx_off; }
+        else {
+            seen.push_back(r);
+            own.push_back(r);
+            D.gx_off = gx_total;
+            gx_total += (long long)D.gx_xb * D.gx_yb * 32 * (D.mesh[2] / 2 + 2 * E.order + 1);
+        }
     }
-    if (changed) CU(cudaMemcpy(E.d.desc, E.desc.data(), sizeof(RepDesc) * E.R, cudaMemcpyHostToDevice));
+    CU(cudaMemcpy(E.d.desc, E.desc.data(), sizeof(RepDesc) * E.R, cudaMemcpyHostToDevice));
+    DALLOC(E.d.gext, (size_t)gx_total);
+    for (int r : own) launch_unfold_octant(E, r, E.stream);
+    CU(cudaGetLastError());
     return PHMC_OK;
 }
 

@@ -27,6 +27,7 @@ struct Engine {
     bool first_stage_off = false;  // the attached surrogate's first stage bypassed (cost-based fallback)
     bool fwd_pipe = false;       // the rebuild's first pass pipelined (persistent blocks, bulk-copied planes)
     int nsm = 0;                 // the device's SM count
+    int run_cluster = 1;         // blocks per replica of the batched Monte Carlo kernel
     float quorum = 0.2f;         // MC launch quorum of blocked replicas (1: every replica runs until it stops)
     cudaStream_t stream = nullptr;
     DevPtrs d{};
@@ -84,6 +85,7 @@ void launch_spread(Engine& E, const int* dirty, cudaStream_t st);
 void launch_fft_pipeline(Engine& E, const int* dirty, int mode, cudaStream_t st);
 void launch_unit_charge(Engine& E, cudaStream_t st);
 void launch_extract_octant(Engine& E, int r, cudaStream_t st);
+void launch_unfold_octant(Engine& E, int r, cudaStream_t st);
 cudaError_t mesh_set_smem_limits(Engine& E);
 
 // k_rebuild.cu
@@ -110,6 +112,9 @@ int sur_train_device(phmc_surrogate* h, const float* d_x, const float* d_sign, c
 enum { MC_RUN = 0, MC_EVAL = 1, MC_APPLY = 2, MC_DESCRIBE = 3, MC_GC = 4 };
 cudaError_t launch_mc(Engine& E, int mode, int rep, const phmc_trial* d_trials, int n, double* d_dE, cudaStream_t st);
 cudaError_t prepare_mc(Engine& E);
+// k_mc_run.cu: plain Monte Carlo, batches of trials per block
+cudaError_t launch_mc_run(Engine& E, cudaStream_t st);
+cudaError_t prepare_mc_run(Engine& E);
 #define GC_EV_BYTES 80  // bytes of one event record of either device phase
 cudaError_t launch_mc_gc(Engine& E, int n_jobs, cudaStream_t st);  // grand-canonical phase: one block per job
 size_t mc_smem_bytes(int order, int pend_max, bool staged_surrogate = false, bool two_buffers = false);

@@ -1,6 +1,10 @@
 // Persistent Monte Carlo kernel: one thread block per replica runs trials
 // back to back until its trial target is reached or its pending-stencil
 // buffer is full (the potential mesh is then rebuilt by the mesh kernels).
+// Runs with the surrogate's first stage or a sample harvest, external trials and
+// the reference's move phases; plain Monte Carlo runs in batches of trials
+// (k_mc_run.cu), which a first stage that ends most trials early, or a proposal
+// stream that depends on the decisions (the reference's generator), does not allow.
 //
 // Per trial (replaces total_energy per trial, MC/src/mc.cu:43-60,241,275,425):
 //  * proposal from a counter-based Philox stream (trial index = counter), so a
@@ -21,20 +25,13 @@
 #include "common.cuh"
 #include "engine.h"
 #include "fft.cuh"
+#include "mc_common.cuh"
 
 #define NST_MAX 4    // stencils per trial
 static_assert(NST_MAX <= 4, "the pair tables count a pending pair's trial stencil by three comparisons");
 #define NPROBE_MAX 4 // (old, new) states of up to two particles
 #define LIST_PF 16   // leading cell-list entries of each probe cell loaded with its count
 #define CAND_MAP 4096 // candidates whose probe-cell entry is tabulated in phase 3
-
-template <int P>
-struct Stencil {
-    int base[3];
-    int m[3][P];   // wrapped mesh coordinates
-    float w[3][P];
-    float coef;
-};
 
 template <int P>
 struct PairK {
@@ -118,33 +115,6 @@ __device__ void trial_setup(TrialS& T, const RepDesc& D) {
         }
     }
     T.nprobe = np; T.nst = ns;
-}
-
-__device__ __forceinline__ float4 rand_pos(const RepDesc& D, uint32_t a, uint32_t b, uint32_t c) {
-    float4 p;
-    p.x = __fmul_rn(D.L[0], u24(a));
-    p.y = __fmul_rn(D.L[1], u24(b));
-    p.z = D.walls ? __fadd_rn(D.wall_lo, __fmul_rn(__fsub_rn(D.wall_hi, D.wall_lo), u24(c))) : __fmul_rn(D.L[2], u24(c));
-    p.w = 0.0f;
-    return p;
-}
-
-// The 16 Philox words of trial t: A = ctr (t, 0), B = ctr (t, 1), C = ctr (t, 2),
-// and ctr (t, 3), whose first two words are the delayed-acceptance first-stage uniform.
-__device__ __forceinline__ void trial_words(const RepDesc& D, long long t, uint32_t* w) {
-    const uint32_t lo = (uint32_t)t, hi = (uint32_t)((unsigned long long)t >> 32);
-    philox4x32_10(D.key[0], D.key[1], lo, hi, 0u, 0u, w);
-    philox4x32_10(D.key[0], D.key[1], lo, hi, 1u, 0u, w + 4);
-    philox4x32_10(D.key[0], D.key[1], lo, hi, 2u, 0u, w + 8);
-    philox4x32_10(D.key[0], D.key[1], lo, hi, 3u, 0u, w + 12);
-}
-
-__device__ __forceinline__ int move_of(const RepDesc& D, uint32_t a0) {
-    const float um = u24(a0);
-    if (um < D.p_disp) return PHMC_MOVE_DISP;
-    if (um < D.p_disp + D.p_titr) return PHMC_MOVE_TITR;
-    if (um < D.p_disp + D.p_titr + D.p_swap) return PHMC_MOVE_SWAP;
-    return PHMC_MOVE_NONE;
 }
 
 // Load the primary particle of trial t into pf (list index from the current sizes).
@@ -325,76 +295,6 @@ __device__ void load_external(TrialS& T, const RepDesc& D, const DevPtrs& d, con
         T.tn[k] = e.c[k].type;
     }
     if (T.nch == 1) T.move = PHMC_MOVE_DISP;
-}
-
-// Axis k of the stencil of a charge at p (weights, base, wrapped mesh indices).
-template <int P>
-__device__ __forceinline__ void make_stencil_axis(Stencil<P>& s, const RepDesc& D, float4 p, int k) {
-    const float pk = (k == 0) ? p.x : (k == 1 ? p.y : p.z);
-    const float g = pk / D.L[k] * (float)D.mesh[k];
-    const float fl = floorf(g);
-    float w[P];
-    bspline_weights<P>(g - fl, w);
-    const int base = (int)fl + P / 2 - P + 1;
-    s.base[k] = base;
-#pragma unroll
-    for (int j = 0; j < P; ++j) {  // base + j lies in [-P, n + P): one correction wraps it
-        int m = base + j;
-        m += (m < 0) ? D.mesh[k] : 0;
-        m -= (m >= D.mesh[k]) ? D.mesh[k] : 0;
-        s.m[k][j] = m;
-        s.w[k][j] = w[j];
-    }
-}
-
-
-__device__ __forceinline__ int wrap1(int i, int n) { return i < 0 ? i + n : (i >= n ? i - n : i); }
-// i mod n for |i| within a few periods (descriptor cell offsets)
-__device__ __forceinline__ int wrap_small(int i, int n) {
-    while (i < 0) i += n;
-    while (i >= n) i -= n;
-    return i;
-}
-
-__device__ __forceinline__ void list_remove(int* list, int* pos, int& n, int so, int i) {
-    const int k = pos[so + i];
-    const int last = list[so + n - 1];
-    list[so + k] = last; pos[so + last] = k;
-    --n;
-    pos[so + i] = -1;
-}
-__device__ __forceinline__ void list_append(int* list, int* pos, int& n, int so, int i) {
-    list[so + n] = i; pos[so + i] = n; ++n;
-}
-
-__device__ bool cell_remove(const DevPtrs& d, const RepDesc& D, int i) {
-    const int gi = D.slot_off + i;
-    const int c = d.cell_of[gi], k = d.cell_pos[gi];
-    int* cnt = d.cell_count + D.cell_off + c;
-    int* l = d.cell_list + ((size_t)D.cell_off + c) * D.cell_cap;
-    const int n = *cnt;
-    const int last = l[n - 1];
-    l[k] = last; d.cell_pos[D.slot_off + last] = k;
-    *cnt = n - 1;
-    d.cell_of[gi] = -1; d.cell_pos[gi] = -1;
-    return true;
-}
-__device__ bool cell_insert(const DevPtrs& d, const RepDesc& D, int i, int c) {
-    const int gi = D.slot_off + i;
-    int* cnt = d.cell_count + D.cell_off + c;
-    const int n = *cnt;
-    if (n >= D.cell_cap) return false;
-    d.cell_list[((size_t)D.cell_off + c) * D.cell_cap + n] = i;
-    *cnt = n + 1;
-    d.cell_of[gi] = c; d.cell_pos[gi] = n;
-    return true;
-}
-
-__device__ __forceinline__ double slab_energy(const RepDesc& D, double Q, double Mz, double S2) {
-    if (!D.slab) return 0.0;
-    double e = D.slab_coef * Mz * Mz;
-    if (fabs(Q) > 1e-4) e -= D.slab_coef * Q * (S2 + Q * D.Lz2_12);
-    return e;
 }
 
 // Charge-moment changes of trial T and the self / net-charge / slab energy changes.
@@ -764,11 +664,6 @@ __device__ int p2_decide(GcDev& G, const RepDesc& D, const RepState& S, const De
     return accept;
 }
 
-// (an atomic add whose result is unused does not wait for the line: the commit thread goes on)
-__device__ __forceinline__ void cls_add(const DevPtrs& d, const RepDesc& D, int cell, int cls, int delta) {
-    if (cls >= 0 && cell >= 0) atomicAdd(reinterpret_cast<int*>(d.cell_cls + D.cell_off + cell) + cls, delta);
-}
-
 template <int NT>
 __device__ __forceinline__ void block_sum3(double& a, double& b, double& c, double* red) {
 #pragma unroll
@@ -794,9 +689,7 @@ __device__ __forceinline__ void block_sum3(double& a, double& b, double& c, doub
 // flight per step of the pending-correction sum (2-4: one row per work item, strided over
 // the block; 20 + w: one pair per warp, w pairs in flight, lanes over the pair's (dy, dx)
 // plane); both tuning parameters
-// FS: the surrogate's first stage (descriptor, network, training-sample harvest) compiled in;
-// launches that use none of it (plain Monte Carlo) take the instance without its code, whose
-// hot loop is then smaller in the instruction caches
+// FS: the surrogate's first stage (descriptor, network, training-sample harvest) compiled in
 template <int P, int NT, bool GC, int RC = 4, int RR = 2, bool FS = true>
 __global__ void __launch_bounds__(NT, 512 / NT) k_mc(DevPtrs d, int mode, int ext_rep, const phmc_trial* __restrict__ ext, int n_ext,
                                            double* __restrict__ ext_dE, int pend_max) {
@@ -846,9 +739,6 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_mc(DevPtrs d, int mode, int ex
     __shared__ int s_gc_ops, s_gc_find, s_gc_lt;
     __shared__ unsigned int s_zh[3 * PHMC_ZHIST_MAX_BINS];
 
-    // the instance without the first stage runs Monte Carlo launches only: with the mode a
-    // constant the external-trial paths drop out of its code as well
-    if constexpr (!FS && !GC) mode = MC_RUN;
     const int r = GC ? d.gc[blockIdx.x].replica : ((mode == MC_RUN) ? blockIdx.x : ext_rep);
     const int tid = threadIdx.x;
     if constexpr (GC) {
@@ -966,33 +856,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_mc(DevPtrs d, int mode, int ex
                 if (wj < s_nqjob) {
                     const float4 pq = s_qjob[wj];
                     const bool neg = s_qsgn[wj] < 0;
-                    float w[3][P];
-                    int base[3];
-                    qmesh_stencil<P>(D, pq, w, base);
-                    const int nx = D.mesh[0], ny = D.mesh[1], nz = D.mesh[2];
-                    unsigned long long* qb = d.qband + D.qb_off;
-                    const int lane = tid & 31;  // lane (bb, c) < P^2 writes the row of P points
-                    const int bb = lane % P, c = lane / P;
-                    int zr = base[2] + c - D.zb_lo;
-                    zr %= nz;
-                    zr += (zr < 0) ? nz : 0;
-                    if (lane < P * P && zr < D.zb_n) {
-                        float wy = 0.0f, wz = 0.0f;  // selects keep the weights in registers
-#pragma unroll
-                        for (int j = 0; j < P; ++j) { wy = (j == bb) ? w[1][j] : wy; wz = (j == c) ? w[2][j] : wz; }
-                        int yb = base[1] + bb;
-                        yb += (yb < 0) ? ny : 0;
-                        yb -= (yb >= ny) ? ny : 0;
-                        unsigned long long* row = qb + ((size_t)zr * ny + yb) * nx;
-#pragma unroll
-                        for (int a = 0; a < P; ++a) {
-                            int xa = base[0] + a;
-                            xa += (xa < 0) ? nx : 0;
-                            xa -= (xa >= nx) ? nx : 0;
-                            const long long v = qmesh_value(pq.w, w[0][a], wy, wz);
-                            atomicAdd(&row[xa], (unsigned long long)(neg ? -v : v));
-                        }
-                    }
+                    qmesh_update<P>(D, d, pq, neg, tid & 31);
                 }
             }
             // idle threads: store the previous trial's harvested rows, clear the shell histogram
@@ -1821,9 +1685,7 @@ template <int P, int NT, int RC, int RR>
 static cudaError_t launch_mc_t(Engine& E, int mode, int rep, const phmc_trial* t, int n, double* dE, cudaStream_t st) {
     DevPtrs dd = E.d;
     if (E.first_stage_off) dd.sur.H = 0;  // surrogate attached but bypassed: every trial exact
-    // plain Monte Carlo (no network, no harvest) takes the instance without the first stage
-    const bool fs = dd.sur.H > 0 || dd.hv_cap > 0 || mode != MC_RUN;
-    auto kern = fs ? k_mc<P, NT, false, RC, RR, true> : k_mc<P, NT, false, RC, RR, false>;
+    auto kern = k_mc<P, NT, false, RC, RR, true>;
     size_t smem = mc_smem_bytes(P, E.pend_max, false);
     dd.sur_late_l3 = 0;
     if (dd.sur.H > 0) {
@@ -1894,17 +1756,13 @@ static cudaError_t prepare_mc_t(Engine& E) {
     int optin = 0;
     cudaError_t e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, E.device);
     if (e != cudaSuccess) return e;
-    for (int fs = 0; fs < 2; ++fs) {  // with and without the first stage
-        auto kern = fs ? k_mc<P, NT, false, RC, RR, true> : k_mc<P, NT, false, RC, RR, false>;
-        cudaFuncAttributes fa;
-        e = cudaFuncGetAttributes(&fa, kern);
-        if (e != cudaSuccess) return e;
-        const int cap = optin - (int)fa.sharedSizeBytes;
-        if ((size_t)cap < mc_smem_bytes(P, E.pend_max, true)) return cudaErrorInvalidValue;
-        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, cap);
-        if (e != cudaSuccess) return e;
-    }
-    return cudaSuccess;
+    auto kern = k_mc<P, NT, false, RC, RR, true>;
+    cudaFuncAttributes fa;
+    e = cudaFuncGetAttributes(&fa, kern);
+    if (e != cudaSuccess) return e;
+    const int cap = optin - (int)fa.sharedSizeBytes;
+    if ((size_t)cap < mc_smem_bytes(P, E.pend_max, true)) return cudaErrorInvalidValue;
+    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, cap);
 }
 
 // The compiled (order, round width, G rows) variants: order 5 (the configurations' order)
@@ -1930,6 +1788,8 @@ static cudaError_t mc_dispatch(const Engine& E, F&& f) {
 }
 
 cudaError_t prepare_mc(Engine& E) {
+    cudaError_t e = prepare_mc_run(E);
+    if (e != cudaSuccess) return e;
     return mc_dispatch(E, [&](auto p, auto nt, auto rc, auto rr) {
         return prepare_mc_t<decltype(p)::value, decltype(nt)::value, decltype(rc)::value, decltype(rr)::value>(E);
     });
@@ -1951,6 +1811,8 @@ size_t mc_smem_bytes(int order, int pend_max, bool staged_surrogate, bool two_bu
 }
 
 cudaError_t launch_mc(Engine& E, int mode, int rep, const phmc_trial* t, int n, double* dE, cudaStream_t st) {
+    // plain Monte Carlo (no network, no harvest) runs in batches of trials (k_mc_run.cu)
+    if (mode == MC_RUN && !(E.d.sur.H > 0 && !E.first_stage_off) && E.d.hv_cap == 0) return launch_mc_run(E, st);
     return mc_dispatch(E, [&](auto p, auto nt, auto rc, auto rr) {
         return launch_mc_t<decltype(p)::value, decltype(nt)::value, decltype(rc)::value, decltype(rr)::value>(
             E, mode, rep, t, n, dE, st);

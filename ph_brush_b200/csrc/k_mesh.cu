@@ -240,6 +240,21 @@ void launch_unit_charge(Engine& E, cudaStream_t st) {
     k_unit_charge<<<(E.R + 127) / 128, 128, 0, st>>>(E.d, E.R);
 }
 
+// The octant unfolded into the blocked table that the batched Monte Carlo kernel reads.
+__global__ void k_unfold_octant(DevPtrs d, int r) {
+    const RepDesc& D = d.desc[r];
+    const int P = D.order;
+    const int ez = D.mesh[2] / 2 + 2 * P + 1;
+    const int plane = D.gx_xb * D.gx_yb * 32;
+    auto fold = [](int c, int n) { c %= n; c += (c < 0) ? n : 0; return min(c, n - c); };
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < (long long)plane * ez; i += (long long)gridDim.x * blockDim.x) {
+        const int z = (int)(i / plane), in = (int)(i - (long long)z * plane);
+        const int blk = in >> 5, x = (blk % D.gx_xb) * 4 + (in & 3), y = (blk / D.gx_xb) * 8 + ((in & 31) >> 2);
+        const int fx = fold(x - P, D.mesh[0]), fy = fold(y - P, D.mesh[1]), fz = fold(z - P, D.mesh[2]);
+        d.gext[D.gx_off + i] = d.goct[D.oct_off + ((size_t)fz * D.oct[1] + fy) * D.oct[0] + fx];
+    }
+}
+void launch_unfold_octant(Engine& E, int r, cudaStream_t st) { k_unfold_octant<<<148, 256, 0, st>>>(E.d, r); }
 void launch_extract_octant(Engine& E, int r, cudaStream_t st) { k_extract_octant<<<148, 256, 0, st>>>(E.d, r); }
 
 // The cap is the device's opt-in maximum (not this engine's need), so that
