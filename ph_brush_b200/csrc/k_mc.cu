@@ -741,6 +741,9 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_mc(DevPtrs d, int mode, int ex
 
     const int r = GC ? d.gc[blockIdx.x].replica : ((mode == MC_RUN) ? blockIdx.x : ext_rep);
     const int tid = threadIdx.x;
+    // judged or described trials leave the state alone: a grid of blocks takes them in turn
+    // (512 trials on 11.7k particles: 3280 us on one block, 19 us on 296)
+    const bool ext_step = mode == MC_EVAL || mode == MC_DESCRIBE;
     if constexpr (GC) {
         const int* src = reinterpret_cast<const int*>(d.gc + blockIdx.x);
         int* dst = reinterpret_cast<int*>(&sG);
@@ -760,7 +763,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_mc(DevPtrs d, int mode, int ex
     if (tid == 0) {
         S = d.state[r];
         s_npend = 0;
-        T.ext_k = 0;
+        T.ext_k = ext_step ? blockIdx.x : 0;
         T.stop = 0;
         s_rng_base = -64;
         pf.valid = 0;
@@ -1080,7 +1083,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_mc(DevPtrs d, int mode, int ex
                 if (mode != MC_RUN) {
                     if (ext_dE) ext_dE[T.ext_k] = (T.skip == 5) ? (T.da ? T.dEs : __longlong_as_double(0x7ff8000000000000ll))
                                                                 : __longlong_as_double(0x7ff0000000000000ll);
-                    T.ext_k++;
+                    T.ext_k += ext_step ? gridDim.x : 1;
                 }
             }
             __syncthreads();
@@ -1525,7 +1528,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_mc(DevPtrs d, int mode, int ex
                 double* o = d.ext_comp + (size_t)T.ext_k * 7;
                 o[0] = dlj; o[1] = T.d_fene; o[2] = dc; o[3] = acc_rec; o[4] = dself; o[5] = dqc; o[6] = dslab;
             }
-            if (mode != MC_RUN) T.ext_k++;
+            if (mode != MC_RUN) T.ext_k += ext_step ? gridDim.x : 1;
             if (accept) {
                 if (mode == MC_RUN) S.acc[T.move]++;
                 const int so = D.slot_off;
@@ -1676,6 +1679,10 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_mc(DevPtrs d, int mode, int ex
             asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t_end));
             S.busy_ns += (long long)(t_end - t_start);
         }
+        if (ext_step) {
+            if (S.error) atomicExch(&d.state[r].error, S.error);
+            return;
+        }
         d.state[r] = S;
         if (s_npend > 0) d.dirty[r] = 1;  // potential mesh is stale: rebuild before the next MC launch
     }
@@ -1699,7 +1706,8 @@ static cudaError_t launch_mc_t(Engine& E, int mode, int rep, const phmc_trial* t
         dd.sur_late_l3 = fits2 ? 0 : 1;
         smem = fits2 ? three : mc_smem_bytes(P, E.pend_max, true, true);
     }
-    const int grid = (mode == MC_RUN) ? E.R : 1;
+    // external trials: committed ones one after the other, others as many at once as are resident
+    const int grid = mode == MC_RUN ? E.R : (mode == MC_APPLY ? 1 : std::min(n, E.nsm * (512 / NT)));
     // launch quorum only when every replica's block is resident from the start (otherwise
     // late blocks would count against a quorum the early ones already reached)
     dd.quorum = 1.0f;
