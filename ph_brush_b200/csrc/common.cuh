@@ -267,34 +267,36 @@ __device__ __forceinline__ void bspline_weights(float t, float* w) {
 // point, every operation rounded as written (no contraction), so that the MC
 // kernel's incremental updates and the full spread give the same integers.
 template <int P>
-__device__ __forceinline__ void qmesh_stencil(const RepDesc& D, float4 pq, float (&w)[3][P], int (&base)[3]) {
-    const float p3[3] = {pq.x, pq.y, pq.z};
+__device__ __forceinline__ void qmesh_axis(float pos, float L, int n_mesh, float (&w)[P], int& base) {
+    const float g = __fmul_rn(__fdiv_rn(pos, L), (float)n_mesh);
+    const float fl = floorf(g);
+    const float t = __fsub_rn(g, fl);
+    float c[P];
+    c[0] = t; c[1] = __fsub_rn(1.0f, t);
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        const float g = __fmul_rn(__fdiv_rn(p3[k], D.L[k]), (float)D.mesh[k]);
-        const float fl = floorf(g);
-        const float t = __fsub_rn(g, fl);
-        float c[P];
-        c[0] = t; c[1] = __fsub_rn(1.0f, t);
+    for (int n = 3; n <= P; ++n) {
+        const float inv = 1.0f / (float)(n - 1);
+        float nc[P];
 #pragma unroll
-        for (int n = 3; n <= P; ++n) {
-            const float inv = 1.0f / (float)(n - 1);
-            float nc[P];
-#pragma unroll
-            for (int i = 0; i < n; ++i) {
-                const float a = (i < n - 1) ? c[i] : 0.0f;
-                const float b = (i >= 1) ? c[i - 1] : 0.0f;
-                const float ta = __fmul_rn(__fadd_rn(t, (float)i), a);
-                const float tb = __fmul_rn(__fsub_rn(__fsub_rn((float)n, t), (float)i), b);
-                nc[i] = __fmul_rn(__fadd_rn(ta, tb), inv);
-            }
-#pragma unroll
-            for (int i = 0; i < n; ++i) c[i] = nc[i];
+        for (int i = 0; i < n; ++i) {
+            const float a = (i < n - 1) ? c[i] : 0.0f;
+            const float b = (i >= 1) ? c[i - 1] : 0.0f;
+            const float ta = __fmul_rn(__fadd_rn(t, (float)i), a);
+            const float tb = __fmul_rn(__fsub_rn(__fsub_rn((float)n, t), (float)i), b);
+            nc[i] = __fmul_rn(__fadd_rn(ta, tb), inv);
         }
 #pragma unroll
-        for (int j = 0; j < P; ++j) w[k][j] = c[P - 1 - j];
-        base[k] = (int)fl + P / 2 - P + 1;
+        for (int i = 0; i < n; ++i) c[i] = nc[i];
     }
+#pragma unroll
+    for (int j = 0; j < P; ++j) w[j] = c[P - 1 - j];
+    base = (int)fl + P / 2 - P + 1;
+}
+template <int P>
+__device__ __forceinline__ void qmesh_stencil(const RepDesc& D, float4 pq, float (&w)[3][P], int (&base)[3]) {
+    qmesh_axis<P>(pq.x, D.L[0], D.mesh[0], w[0], base[0]);
+    qmesh_axis<P>(pq.y, D.L[1], D.mesh[1], w[1], base[1]);
+    qmesh_axis<P>(pq.z, D.L[2], D.mesh[2], w[2], base[2]);
 }
 // q wx wy wz in units of 2^-40 (q wy wz first, as a plane's row weight)
 __device__ __forceinline__ long long qmesh_value(float q, float wx, float wy, float wz) {
@@ -302,6 +304,13 @@ __device__ __forceinline__ long long qmesh_value(float q, float wx, float wy, fl
 }
 
 __device__ __forceinline__ float min_image(float d, float L) { return d - L * rintf(d / L); }
+
+// The same with a product in place of the quotient and the rounding as two adds (exact for
+// |d iL| < 2^22; the quotient and rintf cost a dozen instructions and the slow conversion pipe).
+// The two differ only for offsets near half a box, which lie beyond any cutoff.
+__device__ __forceinline__ float near_image(float d, float L, float iL) {
+    return fmaf(-L, __fadd_rn(__fmaf_rn(d, iL, 12582912.0f), -12582912.0f), d);
+}
 
 __device__ __forceinline__ int wrap_idx(int i, int n) {
     i %= n;

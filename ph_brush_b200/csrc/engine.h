@@ -23,7 +23,7 @@ struct Engine {
     int cand_round = 4;          // pair pass: candidates per thread per round (2, 4, 8 at order 5)
     int g_rows = 2;              // pending-correction sum: G rows in flight per thread (2; 3, 4 with round
                                  // width 2), or 21: one unit of stencil pairs per warp (round width 2 or 4)
-    int energy_block = 128;      // full recompute: particles per block of the pair / FENE pass (0: cell order)
+    int energy_block = 128;      // full recompute: threads per block of the pair / FENE pass (0: 256)
     bool first_stage_off = false;  // the attached surrogate's first stage bypassed (cost-based fallback)
     bool fwd_pipe = false;       // the rebuild's first pass pipelined (persistent blocks, bulk-copied planes)
     int nsm = 0;                 // the device's SM count
@@ -75,7 +75,7 @@ cudaError_t launch_umma_gemm(int M, int N, int K, const __nv_bfloat16* A, long s
                              __nv_bfloat16* Hb, int kchunk, int splits, cudaStream_t st);
 int umma_take_error(cudaStream_t st);
 
-#define PHMC_FULL_MAX_BPR 64  // blocks per replica of the full-recompute pass at most
+#define PHMC_FULL_MAX_BPR 1024  // blocks per replica of the full-recompute pass at most
 
 // engine.cu: records the thread's last error message
 void phmc_set_error(int code, const std::string& msg);

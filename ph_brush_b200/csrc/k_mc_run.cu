@@ -599,8 +599,8 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_mc_run(DevPtrs d, int pend_max
                     for (int p = a.p0; p < a.p0 + a.np && !hit; ++p)
                         for (int q = b.p0; q < b.p0 + b.np; ++q) {
                             const float4 u = B.pp[p], v = B.pp[q];
-                            const float dx = min_image(u.x - v.x, D.L[0]), dy = min_image(u.y - v.y, D.L[1]),
-                                        dz = min_image(u.z - v.z, D.L[2]);
+                            const float dx = near_image(u.x - v.x, D.L[0], s_iL[0]), dy = near_image(u.y - v.y, D.L[1], s_iL[1]),
+                                        dz = near_image(u.z - v.z, D.L[2], s_iL[2]);
                             if (dx * dx + dy * dy + dz * dz <= s_rc2) { hit = true; break; }
                         }
                     for (int k = 0; k < a.nch; ++k)
@@ -683,8 +683,8 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_mc_run(DevPtrs d, int pend_max
                     const int j = hitq[lane];
                     const float4 pj = ld(d.posq + so + j);
                     float elj, ec;
-                    pair_energy(D, min_image(pp.x - pj.x, D.L[0]), min_image(pp.y - pj.y, D.L[1]), min_image(pp.z - pj.z, D.L[2]),
-                                pt, ld(d.type + so + j), pp.w, pj.w, in_bonds(bo, j), elj, ec);
+                    pair_energy(D, near_image(pp.x - pj.x, D.L[0], s_iL[0]), near_image(pp.y - pj.y, D.L[1], s_iL[1]),
+                                near_image(pp.z - pj.z, D.L[2], s_iL[2]), pt, ld(d.type + so + j), pp.w, pj.w, in_bonds(bo, j), elj, ec);
                     alj += (double)(sg * elj);
                     ac += (double)(sg * ec);
                 }
@@ -717,12 +717,9 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_mc_run(DevPtrs d, int pend_max
                     for (int u = 0; u < 2; ++u) {
                         bool hit = false;
                         if (j_u[u] >= 0) {
-                            // (a product in place of min_image's quotient differs only for offsets near
-                            // half a box, which lie beyond any cutoff)
-                            float dx = pp.x - q_u[u].x, dy = pp.y - q_u[u].y, dz = pp.z - q_u[u].z;
-                            dx -= D.L[0] * rintf(dx * s_iL[0]);
-                            dy -= D.L[1] * rintf(dy * s_iL[1]);
-                            dz -= D.L[2] * rintf(dz * s_iL[2]);
+                            const float dx = near_image(pp.x - q_u[u].x, D.L[0], s_iL[0]),
+                                        dy = near_image(pp.y - q_u[u].y, D.L[1], s_iL[1]),
+                                        dz = near_image(pp.z - q_u[u].z, D.L[2], s_iL[2]);
                             hit = dx * dx + dy * dy + dz * dz <= s_rc2;
                         }
                         const unsigned hm = __ballot_sync(0xffffffffu, hit);

@@ -7,6 +7,7 @@
 #include <algorithm>
 #include "common.cuh"
 #include "engine.h"
+#include "fft.cuh"
 
 __global__ void k_cell_assign(DevPtrs d, const int* __restrict__ rep_of, int total) {
     const int gs = blockIdx.x * blockDim.x + threadIdx.x;
@@ -52,143 +53,264 @@ void launch_cell_build(Engine& E, cudaStream_t st) {
 }
 
 #define NCOMP 7
+#define FE_CAND 128  // candidates of a warp at a time
+#define FE_OWN 32    // particles of a cell at a time
+
+// Sums of all pair, bond and charge-moment terms, one warp per cell (cells strided over the
+// grid's warps): the cell's own particles against those of the own cell and of the 13 neighbour
+// cells in the forward half shell, each unordered pair once (with at least 3 cells per axis the 13
+// are distinct).  The warp lists its candidates (one lane per cell for the counts, then one lane
+// per candidate for list entry and particle: two dependent loads in all, where a thread per
+// particle walked 14 cells one after the other) and its lanes take the (own, candidate) pairs.
+// Bound by instruction issue (46 % of the slots: list search, culling, erfc of the ~30 pairs within
+// the cutoff) and those loads' latency.  Measured: 11.7k particles 153 -> 14 us, 64 replicas of 5k
+// 286 -> 191 us, of 8.7k 516 -> 308 us; more warps per SM (fewer registers) were slower.
 template <int NT>
 __global__ void __launch_bounds__(NT) k_full_energy(DevPtrs d, int bpr) {
-    __shared__ double red[40];
-    const int r = blockIdx.y;
-    const RepDesc& D = d.desc[r];
-    double acc[NCOMP] = {0, 0, 0, 0, 0, 0, 0};  // lj, coul, fene(+walls), Q, Q2, Mz, S2
-    for (int i = blockIdx.x * NT + threadIdx.x; i < D.cap; i += bpr * NT) {
-        const int gi = D.slot_off + i;
-        if (d.flags[gi] & PHMC_F_GHOST) continue;
-        const float4 pi = d.posq[gi];
-        const int ti = d.type[gi];
-        const int4 bi = d.bonds[gi];
-        acc[3] += pi.w; acc[4] += (double)pi.w * pi.w;
-        acc[5] += (double)pi.w * pi.z; acc[6] += (double)pi.w * pi.z * pi.z;
-        if (D.walls && (pi.z < D.wall_lo || pi.z >= D.wall_hi)) acc[2] = __longlong_as_double(0x7ff0000000000000ll);
-        const int c = d.cell_of[gi];
-        const int cx = c % D.ncell[0], cy = (c / D.ncell[0]) % D.ncell[1], cz = c / (D.ncell[0] * D.ncell[1]);
-        // each unordered pair once: the own cell with j > i, and every particle of the 13
-        // neighbour cells in the forward half shell (first non-zero offset of (dz, dy, dx)
-        // positive; with at least 3 cells per axis these are 13 distinct cells)
-        for (int h = 0; h < 14; ++h) {
-            const int dz = (h == 0) ? 0 : (h < 5 ? 0 : 1), rem = (h == 0) ? 0 : (h < 5 ? h - 1 : h - 5);
-            int dy, dx;
-            if (h == 0) { dy = 0; dx = 0; }
-            else if (h == 1) { dy = 0; dx = 1; }
-            else if (h < 5) { dy = 1; dx = rem - 2; }            // h = 2..4: (0, 1, -1..1)
-            else { dy = rem / 3 - 1; dx = rem % 3 - 1; }         // h = 5..13: (1, -1..1, -1..1)
-            const int nc = (wrap_idx(cz + dz, D.ncell[2]) * D.ncell[1] + wrap_idx(cy + dy, D.ncell[1])) * D.ncell[0] +
-                           wrap_idx(cx + dx, D.ncell[0]);
-            const int cnt = min(d.cell_count[D.cell_off + nc], D.cell_cap);
-            const int* l = d.cell_list + ((size_t)D.cell_off + nc) * D.cell_cap;
-            for (int k = 0; k < cnt; ++k) {
-                const int j = l[k];
-                if (h == 0 && j <= i) continue;
-                const float4 pj = d.posq[D.slot_off + j];
-                const int tj = d.type[D.slot_off + j];
-                float elj, ec;
-                pair_energy(D, min_image(pi.x - pj.x, D.L[0]), min_image(pi.y - pj.y, D.L[1]),
-                            min_image(pi.z - pj.z, D.L[2]), ti, tj, pi.w, pj.w, in_bonds(bi, j), elj, ec);
-                acc[0] += elj; acc[1] += ec;
-            }
-        }
-        if (D.fene_k > 0.0f) {
-            const int bl[4] = {bi.x, bi.y, bi.z, bi.w};
-            for (int k = 0; k < 4; ++k) {
-                const int j = bl[k];
-                if (j <= i) continue;
-                const float4 pj = d.posq[D.slot_off + j];
-                const float dx = min_image(pi.x - pj.x, D.L[0]), dy = min_image(pi.y - pj.y, D.L[1]), dz = min_image(pi.z - pj.z, D.L[2]);
-                acc[2] += fene_energy(D, dx * dx + dy * dy + dz * dz);
-            }
-        }
-    }
-    for (int k = 0; k < NCOMP; ++k) {
-        const double s = block_sum<NT>(acc[k], red);
-        if (threadIdx.x == 0) d.partials[((size_t)r * bpr + blockIdx.x) * 8 + k] = s;
-    }
-}
-
-// The same sums in cell order: each warp takes whole cells of its replica (cells
-// blockIdx.x * warps + w, strided by the grid), its lanes the cell's particles, and
-// runs over the own cell (partners j > i) and the 13 forward neighbour cells with
-// every lane reading the same partner (one broadcast load per partner instead of
-// 32 divergent walks); particle terms (FENE, walls, charge moments) by the lane that
-// owns the particle.  Per-block partials as k_full_energy, reduced by k_full_reduce.
-template <int NT>
-__global__ void __launch_bounds__(NT) k_full_energy_cells(DevPtrs d, int bpr) {
-    __shared__ double red[40];
     constexpr int NW = NT / 32;
+    __shared__ float4 s_p[NW][FE_CAND], s_o[NW][FE_OWN];
+    __shared__ int s_j[NW][FE_CAND], s_t[NW][FE_CAND], s_ot[NW][FE_OWN];
+    __shared__ int4 s_ob[NW][FE_OWN];
+    __shared__ int s_off[NW][16], s_cell[NW][16];
+    __shared__ int s_hit[NW][64];
+    __shared__ double s_red[NW][NCOMP];
     const int r = blockIdx.y, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const RepDesc& D = d.desc[r];
-    const int ncells = D.ncell[0] * D.ncell[1] * D.ncell[2];
-    double acc[NCOMP] = {0, 0, 0, 0, 0, 0, 0};
-    for (int c = blockIdx.x * NW + w; c < ncells; c += bpr * NW) {
-        const int n = min(d.cell_count[D.cell_off + c], D.cell_cap);
-        if (n == 0) continue;
-        const int cx = c % D.ncell[0], cy = (c / D.ncell[0]) % D.ncell[1], cz = c / (D.ncell[0] * D.ncell[1]);
-        const int* own = d.cell_list + ((size_t)D.cell_off + c) * D.cell_cap;
-        for (int i0 = 0; i0 < n; i0 += 32) {
-            const bool act = i0 + lane < n;
-            const int i = act ? own[i0 + lane] : -1;
-            const int gi = D.slot_off + (act ? i : 0);
-            const float4 pi = act ? d.posq[gi] : make_float4(0.f, 0.f, 0.f, 0.f);
-            const int ti = act ? d.type[gi] : 0;
-            const int4 bi = act ? d.bonds[gi] : make_int4(-1, -1, -1, -1);
-            if (act) {
-                acc[3] += pi.w; acc[4] += (double)pi.w * pi.w;
-                acc[5] += (double)pi.w * pi.z; acc[6] += (double)pi.w * pi.z * pi.z;
-                if (D.walls && (pi.z < D.wall_lo || pi.z >= D.wall_hi)) acc[2] = __longlong_as_double(0x7ff0000000000000ll);
+    // the descriptor in shared memory: an evaluation reads a dozen of its fields
+    __shared__ __align__(16) RepDesc sD;
+    for (int k = threadIdx.x; k < (int)(sizeof(RepDesc) / sizeof(int)); k += NT)
+        reinterpret_cast<int*>(&sD)[k] = reinterpret_cast<const int*>(d.desc + r)[k];
+    __syncthreads();
+    const RepDesc& D = sD;
+    const int nc0 = D.ncell[0], nc1 = D.ncell[1], nc2 = D.ncell[2], cap = D.cell_cap, so = D.slot_off;
+    const int ncells = nc0 * nc1 * nc2;
+    double acc[NCOMP] = {0, 0, 0, 0, 0, 0, 0};  // lj, coul, fene(+walls), Q, Q2, Mz, S2
+    const float Lx = D.L[0], Ly = D.L[1], Lz = D.L[2], iLx = 1.0f / Lx, iLy = 1.0f / Ly, iLz = 1.0f / Lz;
+    // beyond this squared distance two particles have no pair term
+    float rc2 = D.coulomb != PHMC_COUL_NONE ? D.rc_coul2 : 0.0f;
+    for (int k = lane; k < D.T * D.T; k += 32)
+        if (D.lj_eps[k] > 0.0f) rc2 = fmaxf(rc2, D.lj_rc2[k]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) rc2 = fmaxf(rc2, __shfl_xor_sync(0xffffffffu, rc2, o));
+    rc2 *= 1.0001f;
+    int nh = 0;
+    const unsigned below = (1u << lane) - 1u;
+    auto evaluate = [&](int n) {  // the first n (<= 32) queued pairs, one per lane
+        if (lane < n) {
+            const int i = s_hit[w][lane] >> 16, k = s_hit[w][lane] & 0xffff;
+            const float4 pi = s_o[w][i], pj = s_p[w][k];
+            float elj, ec;
+            pair_energy(D, near_image(pi.x - pj.x, Lx, iLx), near_image(pi.y - pj.y, Ly, iLy), near_image(pi.z - pj.z, Lz, iLz), s_ot[w][i], s_t[w][k], pi.w, pj.w, in_bonds(s_ob[w][i], s_j[w][k]), elj, ec);
+            acc[0] += elj; acc[1] += ec;
+        }
+    };
+    auto own_terms = [&](float4 p) {  // single-particle terms
+        acc[3] += p.w; acc[4] += (double)p.w * p.w;
+        acc[5] += (double)p.w * p.z; acc[6] += (double)p.w * p.z * p.z;
+        if (D.walls && (p.z < D.wall_lo || p.z >= D.wall_hi)) acc[2] = __longlong_as_double(0x7ff0000000000000ll);
+    };
+    auto load_partners = [&](int i, float4 p, int4 b, float4 (&pj)[4]) {
+        const int bl[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) pj[k] = bl[k] > i ? d.posq[so + bl[k]] : p;
+    };
+    auto bond_terms = [&](int i, float4 p, int4 b, const float4 (&pj)[4]) {
+        const int bl[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            if (bl[k] <= i) continue;
+            const float dx = min_image(p.x - pj[k].x, Lx), dy = min_image(p.y - pj[k].y, Ly), dz = min_image(p.z - pj[k].z, Lz);
+            acc[2] += fene_energy(D, dx * dx + dy * dy + dz * dz);
+        }
+    };
+    // pairs within the largest cutoff (~15 %) queue up and are evaluated 32 at a time
+    auto near = [&](float4 a, float4 b) {
+        const float dx = near_image(a.x - b.x, Lx, iLx), dy = near_image(a.y - b.y, Ly, iLy), dz = near_image(a.z - b.z, Lz, iLz);
+        return dx * dx + dy * dy + dz * dz <= rc2;
+    };
+    auto push = [&](bool hit, int i, int k) {
+        const unsigned hm = __ballot_sync(0xffffffffu, hit);
+        if (hit) s_hit[w][nh + __popc(hm & below)] = (i << 16) | k;
+        nh += __popc(hm);
+        if (nh >= 32) {
+            __syncwarp();
+            evaluate(32);
+            const int rest = s_hit[w][32 + lane];
+            __syncwarp();
+            s_hit[w][lane] = rest;
+            nh -= 32;
+        }
+    };
+    auto finish = [&]() {  // (the candidates the queue refers to are about to be replaced)
+        __syncwarp();
+        evaluate(nh);
+        nh = 0;
+    };
+    // the 14 cells of c (own cell first), one per lane, and their counts
+    const int hz = lane < 5 ? 0 : 1;
+    const int hy = lane < 2 ? 0 : (lane < 5 ? 1 : (lane - 5) / 3 - 1);
+    const int hx = lane == 0 ? 0 : (lane == 1 ? 1 : (lane < 5 ? lane - 3 : (lane - 5) % 3 - 1));
+    const FastDiv by_x(nc0), by_y(nc1);
+    auto neighbours = [&](int c, int& nc, int& cnt) {
+        nc = 0; cnt = 0;
+        if (lane < 14) {
+            int row, x, y;
+            int z;
+            if (ncells < (1 << 22)) {  // (products of floats are exact enough up to there)
+                row = by_x.div(c, x);
+                z = by_y.div(row, y);
+            } else {
+                row = c / nc0; x = c - row * nc0;
+                z = row / nc1; y = row - z * nc1;
             }
-            for (int h = 0; h < 14; ++h) {
-                const int dz = (h == 0) ? 0 : (h < 5 ? 0 : 1), rem = (h == 0) ? 0 : (h < 5 ? h - 1 : h - 5);
-                int dy, dx;
-                if (h == 0) { dy = 0; dx = 0; }
-                else if (h == 1) { dy = 0; dx = 1; }
-                else if (h < 5) { dy = 1; dx = rem - 2; }
-                else { dy = rem / 3 - 1; dx = rem % 3 - 1; }
-                const int nc = (wrap_idx(cz + dz, D.ncell[2]) * D.ncell[1] + wrap_idx(cy + dy, D.ncell[1])) * D.ncell[0] +
-                               wrap_idx(cx + dx, D.ncell[0]);
-                const int cnt = min(d.cell_count[D.cell_off + nc], D.cell_cap);
-                const int* l = d.cell_list + ((size_t)D.cell_off + nc) * D.cell_cap;
-                for (int k = 0; k < cnt; ++k) {
-                    const int j = l[k];
-                    const float4 pj = d.posq[D.slot_off + j];
-                    const int tj = d.type[D.slot_off + j];
-                    if (!act || (h == 0 && j <= i)) continue;
-                    float elj, ec;
-                    pair_energy(D, min_image(pi.x - pj.x, D.L[0]), min_image(pi.y - pj.y, D.L[1]),
-                                min_image(pi.z - pj.z, D.L[2]), ti, tj, pi.w, pj.w, in_bonds(bi, j), elj, ec);
-                    acc[0] += elj; acc[1] += ec;
-                }
+            x += hx; y += hy; z += hz;
+            x += (x < 0) ? nc0 : (x >= nc0 ? -nc0 : 0);
+            y += (y < 0) ? nc1 : (y >= nc1 ? -nc1 : 0);
+            z -= (z >= nc2) ? nc2 : 0;
+            nc = (z * nc1 + y) * nc0 + x;
+            cnt = min(d.cell_count[D.cell_off + nc], cap);
+        }
+    };
+    const int step = bpr * NW;
+    for (int c0 = blockIdx.x * NW + w; c0 < ncells; c0 += 32 * step) {
+        // the warp's next 32 cells at once: most cells of a padded slab are empty
+        const int cl = c0 + lane * step;
+        unsigned todo = __ballot_sync(0xffffffffu, cl < ncells && d.cell_count[D.cell_off + cl] > 0);
+        int nc = 0, cnt = 0;
+        if (todo) neighbours(c0 + (__ffs(todo) - 1) * step, nc, cnt);
+        while (todo) {
+            const int c = c0 + (__ffs(todo) - 1) * step;
+            todo &= todo - 1;
+            const int n = __shfl_sync(0xffffffffu, cnt, 0);
+            int ofs = cnt;
+#pragma unroll
+            for (int o = 1; o < 16; o <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, ofs, o);
+                if (lane >= o) ofs += y;
             }
-            if (act && D.fene_k > 0.0f) {
-                const int bl[4] = {bi.x, bi.y, bi.z, bi.w};
-                for (int k = 0; k < 4; ++k) {
-                    const int j = bl[k];
-                    if (j <= i) continue;
-                    const float4 pj = d.posq[D.slot_off + j];
-                    const float ddx = min_image(pi.x - pj.x, D.L[0]), ddy = min_image(pi.y - pj.y, D.L[1]),
-                                ddz = min_image(pi.z - pj.z, D.L[2]);
-                    acc[2] += fene_energy(D, ddx * ddx + ddy * ddy + ddz * ddz);
+            const int m = __shfl_sync(0xffffffffu, ofs, 13);
+            __syncwarp();
+            if (lane < 16) { s_off[w][lane] = lane < 14 ? ofs - cnt : 0x7fffffff; s_cell[w][lane] = nc; }
+            __syncwarp();
+            if (todo) neighbours(c0 + (__ffs(todo) - 1) * step, nc, cnt);  // the next cell's, in flight meanwhile
+            auto cell_of = [&](int x) {  // last cell whose offset is <= x
+                int h = 0;
+#pragma unroll
+                for (int st = 8; st > 0; st >>= 1)
+                    if (s_off[w][h + st] <= x) h += st;
+                return h;
+            };
+            if (n <= FE_OWN && m <= FE_CAND) {
+                // usual case: list entries of all candidates, then all particles, each in one round trip;
+                // the own particles are the first n of them
+                int j[FE_CAND / 32];
+                float4 p[FE_CAND / 32];
+                int ty[FE_CAND / 32];
+#pragma unroll
+                for (int u = 0; u < FE_CAND / 32; ++u) {
+                    const int x = lane + 32 * u;
+                    if (x < m) {
+                        const int h = cell_of(x);
+                        j[u] = d.cell_list[((size_t)D.cell_off + s_cell[w][h]) * cap + x - s_off[w][h]];
+                    }
                 }
+#pragma unroll
+                for (int u = 0; u < FE_CAND / 32; ++u)
+                    if (lane + 32 * u < m) { p[u] = d.posq[so + j[u]]; ty[u] = d.type[so + j[u]]; }
+                int4 b = make_int4(-1, -1, -1, -1);
+                if (lane < n) b = d.bonds[so + j[0]];
+#pragma unroll
+                for (int u = 0; u < FE_CAND / 32; ++u)
+                    if (lane + 32 * u < m) { s_j[w][lane + 32 * u] = j[u]; s_p[w][lane + 32 * u] = p[u]; s_t[w][lane + 32 * u] = ty[u]; }
+                float4 pj[4];
+                const bool fene = lane < n && D.fene_k > 0.0f;
+                if (lane < n) {
+                    s_ot[w][lane] = ty[0]; s_o[w][lane] = p[0]; s_ob[w][lane] = b;
+                    if (fene) load_partners(j[0], p[0], b, pj);
+                }
+                __syncwarp();
+                const int mu = (m + 31) / 32;
+                for (int i = 0; i < n; ++i) {
+                    const float4 pi = s_o[w][i];
+#pragma unroll
+                    for (int u = 0; u < FE_CAND / 32; ++u) {
+                        if (u >= mu) break;
+                        const int k = lane + 32 * u;
+                        push(k > i && k < m && near(pi, p[u]), i, k);  // (own cell: later members only)
+                    }
+                }
+                finish();
+                if (lane < n) own_terms(p[0]);
+                if (fene) bond_terms(j[0], p[0], b, pj);
+                __syncwarp();
+                continue;
+            }
+            for (int i0 = 0; i0 < n; i0 += FE_OWN) {
+                const int no = min(n - i0, FE_OWN);
+                if (lane < no) {
+                    const int i = d.cell_list[((size_t)D.cell_off + c) * cap + i0 + lane];
+                    const float4 p = d.posq[so + i];
+                    const int4 b = d.bonds[so + i];
+                    s_ot[w][lane] = d.type[so + i]; s_o[w][lane] = p; s_ob[w][lane] = b;
+                    own_terms(p);
+                    if (D.fene_k > 0.0f) {
+                        float4 pj[4];
+                        load_partners(i, p, b, pj);
+                        bond_terms(i, p, b, pj);
+                    }
+                }
+                for (int base = 0; base < m; base += FE_CAND) {
+                    const int mc = min(m - base, FE_CAND);
+                    __syncwarp();
+                    for (int k = lane; k < mc; k += 32) {
+                        const int x = base + k, h = cell_of(x);
+                        const int j = d.cell_list[((size_t)D.cell_off + s_cell[w][h]) * cap + x - s_off[w][h]];
+                        s_j[w][k] = j; s_p[w][k] = d.posq[so + j]; s_t[w][k] = d.type[so + j];
+                    }
+                    __syncwarp();
+                    for (int i = 0; i < no; ++i)
+                        for (int k0 = 0; k0 < mc; k0 += 32) {
+                            const int k = k0 + lane;
+                            push(k < mc && base + k > i0 + i && near(s_o[w][i], s_p[w][k < mc ? k : 0]), i, k);
+                        }
+                    finish();
+                }
+                __syncwarp();
             }
         }
     }
+#pragma unroll
     for (int k = 0; k < NCOMP; ++k) {
-        const double s = block_sum<NT>(acc[k], red);
-        if (threadIdx.x == 0) d.partials[((size_t)r * bpr + blockIdx.x) * 8 + k] = s;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o);
+        if (lane == 0) s_red[w][k] = acc[k];
+    }
+    __syncthreads();
+    if (threadIdx.x < NCOMP) {
+        double t = 0.0;
+        for (int k = 0; k < NW; ++k) t += s_red[k][threadIdx.x];
+        d.partials[((size_t)r * bpr + blockIdx.x) * 8 + threadIdx.x] = t;
     }
 }
 
-__global__ void k_full_reduce(DevPtrs d, int R, int bpr) {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= R) return;
+// One block per replica: threads over the blocks' partial sums, then over threads, in a fixed order.
+template <int NT>
+__global__ void __launch_bounds__(NT) k_full_reduce(DevPtrs d, int bpr) {
+    __shared__ double s_red[NT / 32][NCOMP];
+    const int r = blockIdx.x, lane = threadIdx.x & 31;
     double a[NCOMP] = {0, 0, 0, 0, 0, 0, 0};
-    for (int b = 0; b < bpr; ++b)
+    for (int b = threadIdx.x; b < bpr; b += NT)
+#pragma unroll
         for (int k = 0; k < NCOMP; ++k) a[k] += d.partials[((size_t)r * bpr + b) * 8 + k];
+#pragma unroll
+    for (int k = 0; k < NCOMP; ++k) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) a[k] += __shfl_xor_sync(0xffffffffu, a[k], o);
+        if (lane == 0) s_red[threadIdx.x >> 5][k] = a[k];
+    }
+    __syncthreads();
+    if (threadIdx.x) return;
+    for (int w = 1; w < NT / 32; ++w)
+        for (int k = 0; k < NCOMP; ++k) a[k] += s_red[w][k];
     const RepDesc& D = d.desc[r];
     RepState& S = d.state[r];
     S.E_pair_lj = a[0]; S.E_pair_c = a[1]; S.E_fene = a[2];
@@ -209,21 +331,16 @@ __global__ void k_full_reduce(DevPtrs d, int R, int bpr) {
     S.E = S.E_pair_lj + S.E_pair_c + S.E_fene + S.E_rec + S.E_self + S.E_qcorr + S.E_slab;
 }
 
-// Particles per block (E.energy_block: 64, 128 or 256; 0 the cell-ordered pass) is a
-// tuning parameter; blocks per replica cover the largest replica, at most
-// PHMC_FULL_MAX_BPR (the partials' size).
+// E.energy_block (64, 128, 256 threads; 0: 256) is a tuning parameter.  Enough blocks per replica
+// for one cell per warp, while all replicas' blocks stay within about four waves of the chip (the
+// rest of the cells in turn); PHMC_FULL_MAX_BPR bounds the partial sums' size.
 void launch_full_energy(Engine& E, cudaStream_t st) {
-    const int nt = E.energy_block;
-    if (nt == 0) {  // cell order: one warp per cell, 8 warps per block
-        const int bpr = std::max(1, std::min(PHMC_FULL_MAX_BPR, (E.max_cells + 7) / 8));
-        k_full_energy_cells<256><<<dim3(bpr, E.R), 256, 0, st>>>(E.d, bpr);
-        k_full_reduce<<<(E.R + 127) / 128, 128, 0, st>>>(E.d, E.R, bpr);
-        return;
-    }
-    const int bpr = std::max(1, std::min(PHMC_FULL_MAX_BPR, (E.max_cap + nt - 1) / nt));
+    const int nt = E.energy_block ? E.energy_block : 256;
+    const int want = (E.max_cells + nt / 32 - 1) / (nt / 32), room = std::max(8, 4 * 148 * 4 * 256 / nt / E.R);
+    const int bpr = std::max(1, std::min({PHMC_FULL_MAX_BPR, want, room}));
     dim3 grid(bpr, E.R);
     if (nt == 64) k_full_energy<64><<<grid, 64, 0, st>>>(E.d, bpr);
     else if (nt == 256) k_full_energy<256><<<grid, 256, 0, st>>>(E.d, bpr);
     else k_full_energy<128><<<grid, 128, 0, st>>>(E.d, bpr);
-    k_full_reduce<<<(E.R + 127) / 128, 128, 0, st>>>(E.d, E.R, bpr);
+    k_full_reduce<128><<<E.R, 128, 0, st>>>(E.d, bpr);
 }
