@@ -30,105 +30,144 @@
 #include "fft.cuh"
 #include "fft_reg.cuh"
 
+// One block per (replica, band plane): the charges whose order-P stencils reach the plane, from the
+// cell list, added into a fixed-point plane in shared memory.  A value (2^-40 units, 41 bits) is
+// added as two 32-bit halves, its low 20 bits and the rest, since 64-bit adds in shared memory are
+// compare-and-swap loops; the halves hold the sums of 4095 charges of 9000 units in all, and a
+// plane that more reach is done over with 64-bit adds.  A warp takes 32 cells at a time, one per
+// lane for the counts, then one lane per member; those that reach the plane (~40 %) queue up and
+// are added 32 at a time: instruction issue bounds it.  Measured on 64 replicas of 8.7k particles: 300 us
+// with 64-bit adds, 262 us as global integer adds, 195 us; one replica of 11.7k: 40 -> 24 us.
 template <int P, int NT>
 __global__ void __launch_bounds__(NT) k_band_spread(DevPtrs d, const int2* __restrict__ jobs) {
     extern __shared__ __align__(16) unsigned char sm_raw[];
+    constexpr int NW = NT / 32;
+    __shared__ float4 s_queue[NW][64];
+    __shared__ int s_n;
+    __shared__ float s_qsum;
     const int2 job = jobs[blockIdx.x];
     const int r = job.x, z = job.y;
     const RepDesc& D = d.desc[r];
-    const int nx = D.mesh[0], ny = D.mesh[1], nz = D.mesh[2];
-    unsigned long long* qp = reinterpret_cast<unsigned long long*>(sm_raw);
-    int* s_cnt = reinterpret_cast<int*>(qp + nx * ny);
-    const int tid = threadIdx.x;
-    for (int i = tid; i < nx * ny; i += NT) qp[i] = 0ull;
-    __syncthreads();
+    const int nx = D.mesh[0], ny = D.mesh[1], nz = D.mesh[2], np = nx * ny;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    float4* queue = s_queue[warp];
+    unsigned* s_lo = reinterpret_cast<unsigned*>(sm_raw);
+    int* s_hi = reinterpret_cast<int*>(sm_raw) + np;
+    unsigned long long* s_64 = reinterpret_cast<unsigned long long*>(sm_raw);
     // floor(g_z) of a contributing charge lies in [z - P/2, z - P/2 + P - 1] (mod nz)
     const float hz = D.L[2] / (float)nz;
-    const float lo = (float)(z - P / 2) * hz, hi = (float)(z - P / 2 + P) * hz;
+    const float zlo = (float)(z - P / 2) * hz, zhi = (float)(z - P / 2 + P) * hz;
     const int ncz = D.ncell[2], ncxy = D.ncell[0] * D.ncell[1];
-    // the cell layers of [lo, hi), widened by a rounding margin (the exact test is per charge)
-    int c_lo = (int)floorf((lo - 1e-3f * hz) * D.cell_scale[2]), c_hi = (int)floorf((hi + 1e-3f * hz) * D.cell_scale[2]);
+    // the cell layers of [zlo, zhi), widened by a rounding margin (the exact test is per charge)
+    int c_lo = (int)floorf((zlo - 1e-3f * hz) * D.cell_scale[2]), c_hi = (int)floorf((zhi + 1e-3f * hz) * D.cell_scale[2]);
     int nlay = c_hi - c_lo + 1;
     if (nlay > ncz) { nlay = ncz; c_lo = 0; }
+    c_lo %= ncz;
+    c_lo += (c_lo < 0) ? ncz : 0;
     const int ncell = nlay * ncxy;
-    // member counts of every cell in the layers, then an exclusive scan, so that the
-    // (cell, member) items spread over all threads with independent loads
-    __shared__ int s_wsum[NT / 32 + 1];
-    // cell of item cc: layer cc / ncxy (wrapped in z), in-layer index cc % ncxy
-    auto cell_of_item = [&](int cc) {
-        const int lay = cc / ncxy, cxy = cc - lay * ncxy;
-        int cz = (c_lo + lay) % ncz;
-        cz += (cz < 0) ? ncz : 0;
-        return cz * ncxy + cxy;
-    };
-    for (int cc = tid; cc < ncell; cc += NT)
-        s_cnt[cc] = min(d.cell_count[D.cell_off + cell_of_item(cc)], D.cell_cap);
-    __syncthreads();
-    {   // block scan: each thread a contiguous chunk, then the chunk totals
-        const int per = (ncell + NT - 1) / NT;
-        const int b0 = min(ncell, tid * per), b1 = min(ncell, b0 + per);
-        int sum = 0;
-        for (int i = b0; i < b1; ++i) sum += s_cnt[i];
-        int x = sum;
-        const int lane = tid & 31, warp = tid >> 5;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, x, o);
-            if (lane >= o) x += y;
-        }
-        if (lane == 31) s_wsum[warp] = x;
+    for (int wide = 0; wide < 2; ++wide) {
+        for (int i = tid; i < np; i += NT) s_64[i] = 0ull;
+        if (tid == 0) { s_n = 0; s_qsum = 0.0f; }
         __syncthreads();
-        if (tid == 0) {
-            int acc = 0;
-            for (int w = 0; w < NT / 32; ++w) { const int v = s_wsum[w]; s_wsum[w] = acc; acc += v; }
-            s_wsum[NT / 32] = acc;
-        }
-        __syncthreads();
-        int run = s_wsum[warp] + x - sum;
-        for (int i = b0; i < b1; ++i) { const int v = s_cnt[i]; s_cnt[i] = run; run += v; }
-        if (tid == NT - 1) s_cnt[ncell] = s_wsum[NT / 32];
-    }
-    __syncthreads();
-    const int total = s_cnt[ncell];
-    for (int it = tid; it < total; it += NT) {
-        int lo2 = 0, hi2 = ncell - 1;  // last cell whose offset <= it
-        while (lo2 < hi2) {
-            const int mid = (lo2 + hi2 + 1) >> 1;
-            if (s_cnt[mid] <= it) lo2 = mid; else hi2 = mid - 1;
-        }
-        const int c = cell_of_item(lo2);
-        const int k = it - s_cnt[lo2];
-        const float4 pq = d.posq[D.slot_off + d.cell_list[((size_t)D.cell_off + c) * D.cell_cap + k]];
-        if (pq.w == 0.0f) continue;
-        float w[3][P];
-        int base[3];
-        qmesh_stencil<P>(D, pq, w, base);
-        int ci = z - base[2];
-        ci %= nz;
-        ci += (ci < 0) ? nz : 0;
-        if (ci >= P) continue;
-        float wz = 0.0f;  // select: w[2][ci] without a dynamic index
+        int n_in = 0, nh = 0;
+        float q_in = 0.0f;
+        auto add = [&](float4 pq) {
+            float w[3][P];
+            int base[3];
+            qmesh_stencil<P>(D, pq, w, base);
+            int ci = z - base[2];
+            ci %= nz;
+            ci += (ci < 0) ? nz : 0;
+            float wz = 0.0f;  // select: w[2][ci] without a dynamic index
 #pragma unroll
-        for (int j = 0; j < P; ++j) wz = (j == ci) ? w[2][j] : wz;
-#pragma unroll
-        for (int bb = 0; bb < P; ++bb) {
-            int yb = base[1] + bb;
-            yb += (yb < 0) ? ny : 0;
-            yb -= (yb >= ny) ? ny : 0;
+            for (int j = 0; j < P; ++j) wz = (j == ci) ? w[2][j] : wz;
+            ++n_in;
+            q_in += fabsf(pq.w);
+            int xa[P];
 #pragma unroll
             for (int aa = 0; aa < P; ++aa) {
-                int xa = base[0] + aa;
-                xa += (xa < 0) ? nx : 0;
-                xa -= (xa >= nx) ? nx : 0;
-                atomicAdd(&qp[yb * nx + xa], (unsigned long long)qmesh_value(pq.w, w[0][aa], w[1][bb], wz));
+                xa[aa] = base[0] + aa;
+                xa[aa] += (xa[aa] < 0) ? nx : 0;
+                xa[aa] -= (xa[aa] >= nx) ? nx : 0;
+            }
+#pragma unroll
+            for (int bb = 0; bb < P; ++bb) {
+                int yb = base[1] + bb;
+                yb += (yb < 0) ? ny : 0;
+                yb -= (yb >= ny) ? ny : 0;
+#pragma unroll
+                for (int aa = 0; aa < P; ++aa) {
+                    const long long v = qmesh_value(pq.w, w[0][aa], w[1][bb], wz);
+                    if (wide) atomicAdd(&s_64[yb * nx + xa[aa]], (unsigned long long)v);
+                    else {
+                        atomicAdd(&s_lo[yb * nx + xa[aa]], (unsigned)(v & 0xfffff));
+                        atomicAdd(&s_hi[yb * nx + xa[aa]], (int)(v >> 20));
+                    }
+                }
+            }
+        };
+        for (int g = warp * 32; g < ncell; g += NW * 32) {
+            const int cc = g + lane;
+            int cell = 0, cnt = 0;
+            if (cc < ncell) {  // layer c_lo + cc / ncxy (wrapped), in-layer index cc % ncxy: consecutive cells
+                cell = c_lo * ncxy + cc;
+                cell -= (cell >= ncz * ncxy) ? ncz * ncxy : 0;
+                cnt = min(d.cell_count[D.cell_off + cell], D.cell_cap);
+            }
+            int ofs = cnt;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, ofs, o);
+                if (lane >= o) ofs += y;
+            }
+            const int m = __shfl_sync(0xffffffffu, ofs, 31);
+            ofs -= cnt;
+            for (int i0 = 0; i0 < m; i0 += 32) {
+                const int i = i0 + lane;
+                int h = 0;  // last cell of the 32 whose offset is <= i
+#pragma unroll
+                for (int st = 16; st > 0; st >>= 1)
+                    if (__shfl_sync(0xffffffffu, ofs, h + st) <= i) h += st;
+                const int hc = __shfl_sync(0xffffffffu, cell, h), ho = __shfl_sync(0xffffffffu, ofs, h);
+                bool hit = false;
+                float4 pq = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (i < m) {
+                    pq = d.posq[D.slot_off + d.cell_list[((size_t)D.cell_off + hc) * D.cell_cap + i - ho]];
+                    if (pq.w != 0.0f) {  // the stencil's first plane, as qmesh_axis has it
+                        int ci = z - ((int)floorf(__fmul_rn(__fdiv_rn(pq.z, D.L[2]), (float)nz)) + P / 2 - P + 1);
+                        ci %= nz;
+                        ci += (ci < 0) ? nz : 0;
+                        hit = ci < P;
+                    }
+                }
+                const unsigned hm = __ballot_sync(0xffffffffu, hit);
+                if (hit) queue[nh + __popc(hm & ((1u << lane) - 1u))] = pq;
+                nh += __popc(hm);
+                if (nh >= 32) {
+                    __syncwarp();
+                    add(queue[lane]);
+                    const float4 rest = queue[32 + lane];
+                    __syncwarp();
+                    if (lane < nh - 32) queue[lane] = rest;
+                    nh -= 32;
+                }
             }
         }
+        __syncwarp();
+        if (lane < nh) add(queue[lane]);
+        if (n_in) { atomicAdd(&s_n, n_in); atomicAdd(&s_qsum, q_in); }
+        __syncthreads();
+        int zrel = z - D.zb_lo;
+        zrel += (zrel < 0) ? nz : 0;
+        unsigned long long* q = d.qband + D.qb_off + (size_t)zrel * np;
+        const bool fits = s_n <= 4095 && s_qsum <= 9000.0f;
+        if (wide || fits) {
+            for (int i = tid; i < np; i += NT)
+                q[i] = wide ? s_64[i] : (unsigned long long)(((long long)s_hi[i] << 20) + (long long)s_lo[i]);
+            return;
+        }
+        __syncthreads();
     }
-    __syncthreads();
-    int zrel = z - D.zb_lo;
-    zrel += (zrel < 0) ? nz : 0;
-    unsigned long long* q = d.qband + D.qb_off + (size_t)zrel * nx * ny;
-    for (int i = tid; i < nx * ny; i += NT) q[i] = qp[i];
 }
 
 template <int NT>
