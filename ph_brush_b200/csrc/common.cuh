@@ -37,15 +37,19 @@ struct GcDev {
     long long s_before, s_after;
     // phase 2 (MC/src/mc.cu:159-318): phase 1 = grand-canonical mu control, 2 = swaps with patience
     int phase;
-    int role;                // 0 next attempt, 1 NH half of a four-point move (applied), 2 judged move, 3 NH half restored
+    int role;                // 0 next attempt, 1 NH half of a four-point move (applied), 2 judged move
     int four;                // the current attempt is a four-point move
     int prefer_wc;
     int max_attempts, patience, energy_interval, since_best;
     float best_E;
     int iP, iN, jCl, jW;     // the attempt's atoms
-    int o_type[2];           // identities of iP, iN before the attempt
-    float o_q[2];
-    int stop_after_restore;  // phase ends once the NH half is restored
+    int k[4];                // their places in the pools (phase 1: NH site, W / Cl partner)
+    // before the NH half was applied: iP's and iN's identities (and their charges with it), slot
+    // flags, pending stencils, tracked energies (RepState's E .. E_slab) and charge moments
+    int o_type[2], o_flags[2], o_npend;
+    float4 o_pq[2];
+    float n_q[2];
+    double o_E[8], o_mom[4];
     int fixed;               // mu held fixed: no feedback, no target stop
 };
 

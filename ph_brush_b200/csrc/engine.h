@@ -27,6 +27,7 @@ struct Engine {
     bool first_stage_off = false;  // the attached surrogate's first stage bypassed (cost-based fallback)
     bool fwd_pipe = false;       // the rebuild's first pass pipelined (persistent blocks, bulk-copied planes)
     int nsm = 0;                 // the device's SM count
+    size_t mc512_smem = 0;       // dynamic shared memory the 512-thread first-stage kernel is prepared for
     int run_cluster = 1;         // blocks per replica of the batched Monte Carlo kernel
     float quorum = 0.2f;         // MC launch quorum of blocked replicas (1: every replica runs until it stops)
     cudaStream_t stream = nullptr;

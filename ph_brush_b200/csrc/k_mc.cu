@@ -26,22 +26,12 @@
 #include "engine.h"
 #include "fft.cuh"
 #include "mc_common.cuh"
+#include "mc_window.cuh"
 
 #define NST_MAX 4    // stencils per trial
-static_assert(NST_MAX <= 4, "the pair tables count a pending pair's trial stencil by three comparisons");
 #define NPROBE_MAX 4 // (old, new) states of up to two particles
 #define LIST_PF 16   // leading cell-list entries of each probe cell loaded with its count
 #define CAND_MAP 4096 // candidates whose probe-cell entry is tabulated in phase 3
-
-template <int P>
-struct PairK {
-    float K[3][2 * P - 1];
-    int f[3][2 * P - 1];  // folded octant coordinate of D + delta
-    float coef;
-    int pad;
-    // (row offsets and coef * Ky * Kz are recomputed where they are used: 224 bytes per
-    // pair at order 5 keep two MC blocks per SM up to ~100 pending stencils)
-};
 
 struct TrialS {
     int stop, skip, move, nch, accept, nprobe, nst, ext_k;
@@ -57,7 +47,7 @@ struct TrialS {
     float4 st_pos[NST_MAX];
     float st_coef[NST_MAX];
     double d_direct_lj, d_direct_c, d_fene;
-    int total_cand, npairs;
+    int total_cand;
     // cell bookkeeping of the old states, loaded off the critical path (phase 4)
     int cell_old[2], cpos_old[2], cnt_old[2], last_old[2];
     int fo[2];  // slot flags of the changed particles before the trial
@@ -434,8 +424,10 @@ __device__ void gc_propose(TrialS& T, GcDev& G, const RepDesc& D, const DevPtrs&
         T.stop = 1;
         return;
     }
-    const int i = gc_pool(d, D, fwd ? GC_NHN : GC_NHP)[mt_index(G.mt, (uint32_t)(fwd ? a : b))];
-    const int j = gc_pool(d, D, fwd ? GC_W : GC_CL)[mt_index(G.mt, (uint32_t)(fwd ? c : e))];
+    const int ki = (int)mt_index(G.mt, (uint32_t)(fwd ? a : b)), kj = (int)mt_index(G.mt, (uint32_t)(fwd ? c : e));
+    const int i = gc_pool(d, D, fwd ? GC_NHN : GC_NHP)[ki];
+    const int j = gc_pool(d, D, fwd ? GC_W : GC_CL)[kj];
+    G.k[0] = ki; G.k[1] = kj;
     G.dir = fwd ? 1 : -1;
     G.s_before = wf + wb;
     G.s_after = fwd ? (a - 1) * (c - 1) + (b + 1) * (e + 1) : (a + 1) * (c + 1) + (b - 1) * (e - 1);
@@ -516,27 +508,30 @@ __device__ int gc_decide(GcDev& G, const RepDesc& D, const RepState& S, const De
     return accept;
 }
 
-// Move slot v from pool src to the end of pool dst, keeping the order of the rest
-// (std::vector erase + push_back); all threads of the block.
+// Move entry k0 (slot v) of pool src to the end of pool dst, keeping the order of the rest
+// (std::vector erase + push_back); all threads of the block, eight entries each per step (the
+// proposal knows the entry: a search over the pool and a step per NT entries took four times as long).
 template <int NT>
-__device__ void gc_pool_move(int* src, int* dst, int& n_src, int& n_dst, int v, int* s_find) {
-    if (threadIdx.x == 0) *s_find = 0x7fffffff;
-    __syncthreads();
+__device__ void gc_pool_move(int* src, int* dst, int& n_src, int& n_dst, int v, int k0) {
+    constexpr int U = 8;
     const int n = n_src;
-    for (int k = threadIdx.x; k < n; k += NT)
-        if (src[k] == v) atomicMin(s_find, k);
-    __syncthreads();
-    const int k0 = *s_find;
-    if (k0 < n) {
-        for (int b = k0; b < n - 1; b += NT) {  // shift the tail down by one, NT entries per step
-            const int k = b + threadIdx.x;
-            const int val = (k < n - 1) ? src[k + 1] : 0;
-            __syncthreads();
-            if (k < n - 1) src[k] = val;
-            __syncthreads();
+    for (int b = k0; b < n - 1; b += U * NT) {
+        int val[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int k = b + u * NT + threadIdx.x;
+            val[u] = (k < n - 1) ? src[k + 1] : 0;
         }
-        if (threadIdx.x == 0) { dst[n_dst] = v; n_dst = n_dst + 1; n_src = n - 1; }
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int k = b + u * NT + threadIdx.x;
+            if (k < n - 1) src[k] = val[u];
+        }
+        __syncthreads();
     }
+    __syncthreads();
+    if (threadIdx.x == 0) { dst[n_dst] = v; n_dst = n_dst + 1; n_src = n - 1; }
     __syncthreads();
 }
 
@@ -553,8 +548,7 @@ __device__ __forceinline__ void p2_change(TrialS& T, const DevPtrs& d, const Rep
 
 // Next two-atom evaluation of phase 2 (one thread).  An attempt draws its atoms in the
 // reference's order (NH_P, NH_N, Cl, W; or Cl, W) and starts with the NH half of a
-// four-point move, or is a Cl/W move; the Cl/W half follows; a rejected four-point
-// move ends with the NH half restored.  Attempts start only with room for all of their
+// four-point move, or is a Cl/W move; the Cl/W half follows.  Attempts start only with room for all of their
 // pending stencils, so a launch never ends inside one.
 __device__ void p2_propose(TrialS& T, GcDev& G, const RepDesc& D, const DevPtrs& d, int npend, int pend_max, int& launch_trials) {
     T.move = PHMC_MOVE_NONE; T.skip = 0; T.nch = 2; T.logf = 0.0; T.tnum = G.attempted;
@@ -562,12 +556,6 @@ __device__ void p2_propose(TrialS& T, GcDev& G, const RepDesc& D, const DevPtrs&
         p2_change(T, d, D, 0, G.jCl, G.type[GC_W], 0.0f);
         p2_change(T, d, D, 1, G.jW, G.type[GC_CL], G.q_cl);
         G.role = 2; ++launch_trials;
-        return;
-    }
-    if (G.role == 3) {  // restore the NH half of the rejected move
-        p2_change(T, d, D, 0, G.iP, G.o_type[0], G.o_q[0]);
-        p2_change(T, d, D, 1, G.iN, G.o_type[1], G.o_q[1]);
-        ++launch_trials;
         return;
     }
     if (G.stop || launch_trials >= G.launch_cap) { T.stop = 1; return; }
@@ -583,23 +571,28 @@ __device__ void p2_propose(TrialS& T, GcDev& G, const RepDesc& D, const DevPtrs&
         G.stop = PHMC_P2_STOP_NO_PROPOSALS; T.stop = 1;
         return;
     }
-    if (npend + (four ? 6 : 2) > pend_max) { T.stop = 1; return; }
+    if (npend + (four ? 4 : 2) > pend_max) { T.stop = 1; return; }
     G.attempted++;
     G.four = four ? 1 : 0;
-    const int so = D.slot_off;
     if (four) {
-        G.iP = gc_pool(d, D, GC_NHP)[mt_index(G.mt, (uint32_t)G.n[GC_NHP])];
-        G.iN = gc_pool(d, D, GC_NHN)[mt_index(G.mt, (uint32_t)G.n[GC_NHN])];
-        G.jCl = gc_pool(d, D, GC_CL)[mt_index(G.mt, (uint32_t)G.n[GC_CL])];
-        G.jW = gc_pool(d, D, GC_W)[mt_index(G.mt, (uint32_t)G.n[GC_W])];
-        G.o_type[0] = d.type[so + G.iP]; G.o_q[0] = d.posq[so + G.iP].w;
-        G.o_type[1] = d.type[so + G.iN]; G.o_q[1] = d.posq[so + G.iN].w;
+        // the draws first, then the four entries in one round trip
+        const int kP = (int)mt_index(G.mt, (uint32_t)G.n[GC_NHP]), kN = (int)mt_index(G.mt, (uint32_t)G.n[GC_NHN]);
+        const int kC = (int)mt_index(G.mt, (uint32_t)G.n[GC_CL]), kW = (int)mt_index(G.mt, (uint32_t)G.n[GC_W]);
+        const int iP = gc_pool(d, D, GC_NHP)[kP], iN = gc_pool(d, D, GC_NHN)[kN];
+        const int jCl = gc_pool(d, D, GC_CL)[kC], jW = gc_pool(d, D, GC_W)[kW];
+        G.iP = iP; G.iN = iN; G.jCl = jCl; G.jW = jW;
+        G.k[0] = kP; G.k[1] = kN; G.k[2] = kC; G.k[3] = kW;
         p2_change(T, d, D, 0, G.iP, G.type[GC_NHN], 0.0f);
         p2_change(T, d, D, 1, G.iN, G.type[GC_NHP], G.q_nhp);
+        for (int k = 0; k < 2; ++k) {
+            G.o_type[k] = T.to[k]; G.o_flags[k] = T.fo[k]; G.o_pq[k] = T.po[k]; G.n_q[k] = T.pn[k].w;
+        }
         G.role = 1;
     } else {
-        G.jCl = gc_pool(d, D, GC_CL)[mt_index(G.mt, (uint32_t)G.n[GC_CL])];
-        G.jW = gc_pool(d, D, GC_W)[mt_index(G.mt, (uint32_t)G.n[GC_W])];
+        const int kC = (int)mt_index(G.mt, (uint32_t)G.n[GC_CL]), kW = (int)mt_index(G.mt, (uint32_t)G.n[GC_W]);
+        const int jCl = gc_pool(d, D, GC_CL)[kC], jW = gc_pool(d, D, GC_W)[kW];
+        G.jCl = jCl; G.jW = jW;
+        G.k[2] = kC; G.k[3] = kW;
         p2_change(T, d, D, 0, G.jCl, G.type[GC_W], 0.0f);
         p2_change(T, d, D, 1, G.jW, G.type[GC_CL], G.q_cl);
         G.role = 2;
@@ -607,18 +600,22 @@ __device__ void p2_propose(TrialS& T, GcDev& G, const RepDesc& D, const DevPtrs&
     ++launch_trials;
 }
 
-// Decision of a phase-2 evaluation (one thread).  The NH half and its restoration are
-// applied unconditionally; the judged move follows the reference (MC/src/mc.cu:241-293):
+// Decision of a phase-2 evaluation (one thread).  The NH half is applied unconditionally, with
+// what it changes kept so that a rejected move takes it back without an evaluation (undo; as a
+// third evaluation it cost half as much again and left four pending stencils that cancel: 100
+// attempts on 14.9k particles: 10 launches and rebuilds where there are 3 now); the judged move follows the
+// reference (MC/src/mc.cu:241-293):
 // dE from the reference's float energies, accepted if dE <= 0 or exp(clamp(-beta dE))
 // beats a uniform draw; then the best-energy / patience bookkeeping and the report line.
 // Returns the decision; *pool_ops gets 2 (four-point pools), 3 (Cl/W pools) or 0.
-__device__ int p2_decide(GcDev& G, const RepDesc& D, const RepState& S, const DevPtrs& d, double dlj, double dc, double drec,
-                         double dself, double dqc, double dslab, int* pool_ops) {
+__device__ int p2_decide(GcDev& G, const RepDesc& D, const RepState& S, const DevPtrs& d, int npend, double dlj, double dc,
+                         double drec, double dself, double dqc, double dslab, int* pool_ops, int* undo) {
     *pool_ops = 0;
-    if (G.role == 1) return 1;  // the NH half: applied, judged with the Cl/W half
-    if (G.role == 3) {          // restored
-        G.role = 0;
-        if (G.stop_after_restore) G.stop = G.stop_after_restore;
+    *undo = 0;
+    if (G.role == 1) {  // the NH half: applied, judged with the Cl/W half
+        G.o_npend = npend;
+        for (int k = 0; k < 8; ++k) G.o_E[k] = (&S.E)[k];
+        for (int k = 0; k < 4; ++k) G.o_mom[k] = (&S.Q)[k];
         return 1;
     }
     const double lj = S.E_pair_lj + dlj;
@@ -639,7 +636,8 @@ __device__ int p2_decide(GcDev& G, const RepDesc& D, const RepState& S, const De
         G.role = 0;
     } else {
         ++G.since_best;
-        G.role = G.four ? 3 : 0;
+        *undo = G.four;
+        G.role = 0;
     }
     if (G.attempted % max(1, G.energy_interval) == 0) {
         phmc_phase2_event ev;
@@ -658,8 +656,7 @@ __device__ int p2_decide(GcDev& G, const RepDesc& D, const RepState& S, const De
         ev.kind = PHMC_P2_EV_PATIENCE;
         ev.since_best = G.since_best; ev.patience = G.patience;
         gc_event(G, d, ev);
-        if (G.role == 3) G.stop_after_restore = PHMC_P2_STOP_PATIENCE;  // the rejected move is undone first
-        else G.stop = PHMC_P2_STOP_PATIENCE;
+        G.stop = PHMC_P2_STOP_PATIENCE;
     }
     return accept;
 }
@@ -684,22 +681,25 @@ __device__ __forceinline__ void block_sum3(double& a, double& b, double& c, doub
     a = red[96]; b = red[97]; c = red[98];
 }
 
+// pending stencils, and those of the trial (external trials: at most NST_MAX, with none pending)
+template <int P>
+__host__ __device__ constexpr size_t mc_stencil_bytes(int pend_max) {
+    return (sizeof(PadSt<P>) * (pend_max + NST_MAX) + 15) / 16 * 16;
+}
+
 // RC: candidate particles per thread and round of the pair pass (the neighbour tile of a
-// round is RC x NT candidates); RR: rows of the influence kernel G each thread has in
-// flight per step of the pending-correction sum (2-4: one row per work item, strided over
-// the block; 20 + w: one pair per warp, w pairs in flight, lanes over the pair's (dy, dx)
-// plane); both tuning parameters
+// round is RC x NT candidates), a tuning parameter
 // FS: the surrogate's first stage (descriptor, network, training-sample harvest) compiled in
-template <int P, int NT, bool GC, int RC = 4, int RR = 2, bool FS = true>
+template <int P, int NT, bool GC, int RC = 4, bool FS = true>
 __global__ void __launch_bounds__(NT, 512 / NT) k_mc(DevPtrs d, int mode, int ext_rep, const phmc_trial* __restrict__ ext, int n_ext,
                                            double* __restrict__ ext_dE, int pend_max) {
-    constexpr int W = 2 * P - 1;
     constexpr int P3 = P * P * P;
+    constexpr int NW = NT / 32;
     extern __shared__ __align__(16) unsigned char dsm[];
     // pending stencils [0, s_npend) followed by the current trial's stencils (a
-    // commit just advances s_npend); then the stencil-pair tables
-    Stencil<P>* s_pend = reinterpret_cast<Stencil<P>*>(dsm);
-    PairK<P>* s_pair = reinterpret_cast<PairK<P>*>(s_pend + pend_max + NST_MAX);
+    // commit just advances s_npend); then each warp's window tables
+    PadSt<P>* s_pend = reinterpret_cast<PadSt<P>*>(dsm);
+    float* s_tab = reinterpret_cast<float*>(dsm + mc_stencil_bytes<P>(pend_max));
     __shared__ TrialS T;
     __shared__ RepState S;
     __shared__ int s_cnt[NPROBE_MAX * 27], s_off[NPROBE_MAX * 27 + 1], s_cell[NPROBE_MAX * 27];
@@ -725,8 +725,8 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_mc(DevPtrs d, int mode, int ex
     __shared__ int s_sfail;                      // a staged copy did not arrive in time
     __shared__ float s_mu[SUR_K], s_sd[SUR_K];   // the attached network's input standardisation
     __shared__ uint16_t s_w4[SUR_HMAX];          // its output weights
-    // staged first stage (aliases the pair tables, used before phase 3): activations, weights
-    unsigned char* sur_base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(s_pair) + 127) & ~uintptr_t(127));
+    // staged first stage (aliases the window tables, used before phase 3): activations, weights
+    unsigned char* sur_base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(s_tab) + 127) & ~uintptr_t(127));
     __nv_bfloat16* act0 = reinterpret_cast<__nv_bfloat16*>(sur_base);
     __nv_bfloat16* act1 = act0 + 16 * SUR_AST;
     uint2* wa = reinterpret_cast<uint2*>(sur_base + SUR_ACT_BYTES);
@@ -736,7 +736,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_mc(DevPtrs d, int mode, int ex
     uint32_t sur_par = 0;  // parity of the weight barriers' current phase (one phase per evaluated move)
     // grand-canonical mu-control phase: the job's state (block blockIdx.x runs job blockIdx.x)
     __shared__ __align__(16) typename std::conditional<GC, GcDev, int>::type sG;
-    __shared__ int s_gc_ops, s_gc_find, s_gc_lt;
+    __shared__ int s_gc_ops, s_gc_lt;
     __shared__ unsigned int s_zh[3 * PHMC_ZHIST_MAX_BINS];
 
     const int r = GC ? d.gc[blockIdx.x].replica : ((mode == MC_RUN) ? blockIdx.x : ext_rep);
@@ -1092,7 +1092,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_mc(DevPtrs d, int mode, int ex
         }
         // ---------------- phase 2: cell counts, stencils, direct & bonded terms ----------------
         const int nent = T.nprobe * 27;
-        Stencil<P>* s_tst = s_pend + s_npend;  // this trial's stencils
+        PadSt<P>* s_tst = s_pend + s_npend;  // this trial's stencils
         if (tid < nent) {
             const int p = tid / 27, nb = tid % 27;
             // the probe's cell coordinates as cell_index computes them (no integer divisions)
@@ -1126,7 +1126,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_mc(DevPtrs d, int mode, int ex
         // the trial's stencils: one thread per (stencil, axis)
         if (tid >= ST0 && tid < ST0 + 3 * T.nst) {
             const int k = (tid - ST0) / 3, ax = tid - ST0 - 3 * k;
-            make_stencil_axis<P>(s_tst[k], D, T.st_pos[k], ax);
+            pad_stencil_axis<P>(s_tst[k], D, T.st_pos[k], ax);
             if (ax == 0) s_tst[k].coef = T.st_coef[k];
         }
         if (tid == DIR) {
@@ -1182,7 +1182,8 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_mc(DevPtrs d, int mode, int ex
         }
         __syncthreads();
         mark(2);
-        // ---------------- phase 3: candidate offsets, stencil pair kernels ----------------
+        // ---------------- phase 3: candidate offsets (warp 0), mesh terms (the other warps) ----------------
+        double acc_lj = 0.0, acc_c = 0.0, acc_rec = 0.0;
         if (tid < 32) {
             int carry = 0;
             for (int b0 = 0; b0 < nent; b0 += 32) {
@@ -1207,49 +1208,46 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_mc(DevPtrs d, int mode, int ex
                 const int b = s_off[e], en = min(s_off[e + 1], CAND_MAP);
                 for (int c = b; c < en; ++c) s_cmap[c] = (uint8_t)e;
             }
-        } else if (D.coulomb == PHMC_COUL_EWALD) {
-            const int nst = T.nst, np = s_npend;
-            const int npairs = nst * np + nst * (nst + 1) / 2;
-            constexpr int W = 2 * P - 1;
-            // one (pair, axis, offset) element per work item
-            for (int e = tid - 32; e < 3 * W * npairs; e += NT - 32) {
-                const int q = e / (3 * W), r3 = e - q * (3 * W);
-                const int k = r3 / W, t = r3 - k * W;
-                int ta, tb;
-                const Stencil<P>* sb;
-                float c;
-                if (q < nst * np) {
-                    ta = (q >= np) + (q >= 2 * np) + (q >= 3 * np);  // q / np for nst <= NST_MAX = 4
-                    tb = q - ta * np;
-                    sb = &s_pend[tb];
-                    c = s_tst[ta].coef * s_pend[tb].coef;
-                } else {
-                    int rem = q - nst * np;
-                    ta = 0;
-                    while (rem >= nst - ta) { rem -= nst - ta; ++ta; }
-                    tb = ta + rem;
-                    sb = &s_tst[tb];
-                    c = s_tst[ta].coef * s_tst[tb].coef * (ta == tb ? 0.5f : 1.0f);
-                }
-                const Stencil<P>& sa = s_tst[ta];
-                const int delta = t - (P - 1);
-                float s = 0.0f;
-#pragma unroll
-                for (int i = 0; i < P; ++i) {
-                    const int j = i - delta;
-                    if (j >= 0 && j < P) s += sa.w[k][i] * sb->w[k][j];
-                }
-                const int n = D.mesh[k];
-                int m = sa.base[k] - sb->base[k] + delta;
-                m += (m < 0) ? n : 0;
-                m += (m < 0) ? n : 0;
-                m -= (m >= n) ? n : 0;
-                m -= (m >= n) ? n : 0;
-                s_pair[q].K[k][t] = s;
-                s_pair[q].f[k][t] = min(m, n - m);
-                if (r3 == 0) s_pair[q].coef = c;
+        } else if (D.coulomb == PHMC_COUL_EWALD && T.nst > 0) {
+            const int nst = T.nst, np = s_npend, warp = (tid >> 5) - 1;
+            // W_t . phi: element (stencil, c, b, a), a fastest (lanes read consecutive x)
+            const float* phi = d.phi + D.mesh_off;
+            const int nx = D.mesh[0], ny = D.mesh[1];
+            for (int it = tid - 32; it < nst * P3; it += NT - 32) {
+                const int st = it / P3, rem = it - st * P3;
+                const int c = rem / (P * P), rb = rem - c * (P * P);
+                const int b = rb / P, a = rb - b * P;
+                const PadSt<P>& s = s_tst[st];
+                const float v = phi[((size_t)s.m[2][c] * ny + s.m[1][b]) * nx + s.m[0][a]];
+                acc_rec += (double)(s.coef * s.wp[0][P + a] * s.wp[1][P + b] * s.wp[2][P + c] * v);
             }
-            if (tid == 32) T.npairs = npairs;
+            // its stencils with every pending one and with one another (half of the diagonal), a
+            // window of G per warp; lanes keep their sums until the block's reduction
+            const float* G = d.gext + D.gx_off;
+            float* tab = s_tab + warp * 2 * Win<P>::TAB;
+            LaneSt<P> L;
+            lane_place<P>(L, D, tid & 31);
+            if (nst <= 2) {
+                lane_stencils<P>(L, D, s_tst, nst);
+                for (int e = warp; e < np + nst; e += NW - 1) {
+                    const PadSt<P>& sb = s_pend[e];
+                    const float c0 = (e == np ? 0.5f : 1.0f) * L.coef0 * sb.coef, c1 = (e == np + 1 ? 0.5f : 1.0f) * L.coef1 * sb.coef;
+                    int w = L.near && e <= np ? 2 : (e == np + 1 ? 1 : 0);
+                    for (;;) {  // both at once, or one after the other
+                        const bool done = window_sum<P>(D, G, L, sb, w, c0, c1, tab, tid & 31, acc_rec);
+                        if (!done) { w = 0; continue; }
+                        if (w == 0 && nst == 2) { w = 1; continue; }
+                        break;
+                    }
+                }
+            } else {  // external trials of two displaced particles: nothing is pending
+                for (int u = warp; u < nst * nst; u += NW - 1) {
+                    const int a = u / nst, b = u - a * nst;
+                    if (b < a) continue;
+                    lane_stencils<P>(L, D, s_tst + a, 1);
+                    window_sum<P>(D, G, L, s_tst[b], 0, (a == b ? 0.5f : 1.0f) * s_tst[a].coef * s_tst[b].coef, 0.0f, tab, tid & 31, acc_rec);
+                }
+            }
         }
         __syncthreads();
         mark(3);
@@ -1280,7 +1278,6 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_mc(DevPtrs d, int mode, int ex
                 T.last_old[k] = (cnt > 0) ? d.cell_list[((size_t)D.cell_off + c) * D.cell_cap + cnt - 1] : -1;
             }
         }
-        double acc_lj = 0.0, acc_c = 0.0, acc_rec = 0.0;
         // quorum of the launch: read here, compared after the pair work (the loads' latency
         // hides behind it), used from the next trial's proposal on
         const bool q_chk = tid == 32 && s_qin;
@@ -1341,118 +1338,6 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_mc(DevPtrs d, int mode, int ex
             __syncthreads();
             mark(4);
         }
-        if (D.coulomb == PHMC_COUL_EWALD) {
-            // W_t . phi: element (stencil, c, b, a), a fastest (lanes read consecutive x)
-            const float* phi = d.phi + D.mesh_off;
-            const int nx = D.mesh[0], ny = D.mesh[1];
-            constexpr int P3 = P * P * P;
-            const int nphi = T.nst * P3;
-            for (int it = tid; it < nphi; it += NT) {
-                const int st = it / P3, rem = it - st * P3;
-                const int c = rem / (P * P), rb = rem - c * (P * P);
-                const int b = rb / P, a = rb - b * P;
-                const Stencil<P>& s = s_tst[st];
-                const float v = phi[((size_t)s.m[2][c] * ny + s.m[1][b]) * nx + s.m[0][a]];
-                acc_rec += (double)(s.coef * s.w[0][a] * s.w[1][b] * s.w[2][c] * v);
-            }
-            // S(W_a, W_b) = sum over (dz, dy) rows of coef Ky Kz sum_dx Kx G[fz, fy, fx]: one
-            // (pair, row) per thread and step, RR rows in flight, the row's W loads back to back;
-            // row sums in FP32 (W terms of one sign pattern), the total in FP64
-            const float* G = d.goct + D.oct_off;
-            const int ox = D.oct[0], oy = D.oct[1];
-            constexpr int WW = W * W;
-            if constexpr (RR > 20) {
-                // one work unit per warp and step: each lane takes EL elements (dy, dx) of the
-                // unit's W x W window plane, so a load instruction reads about 32 / W consecutive
-                // rows of G; the lane's loads of all W z planes are in flight together; FP32 sums
-                // over the lane's EL elements, FP64 over planes.  A unit is one stencil pair, or,
-                // when the trial's two stencils (a displacement's old and new charge) have the
-                // same base, both of its pairs with one pending stencil: their windows are the
-                // same G values (equal folded coordinates), read once and weighted twice
-                static_assert(RR == 21, "one unit in flight per warp");
-                constexpr int EL = (WW + 31) / 32;
-                const int warp = tid >> 5, lane = tid & 31;
-                const int npairs = T.npairs, np = s_npend;
-                const bool merge = T.nst == 2 && np > 0 && s_tst[0].base[0] == s_tst[1].base[0] &&
-                                   s_tst[0].base[1] == s_tst[1].base[1] && s_tst[0].base[2] == s_tst[1].base[2];
-                const int nunit = merge ? npairs - np : npairs;
-                const int oxy = oy * ox;
-                for (int u = warp; u < nunit; u += NT / 32) {
-                    // pairs (trial stencil 0, pending u) and (trial stencil 1, pending u) sit at u
-                    // and np + u of the tables; the trial stencils' own pairs follow at 2 np
-                    const int qa = (merge && u >= np) ? u + np : u;
-                    const int qb = (merge && u < np) ? np + u : -1;
-                    const PairK<P>& pa = s_pair[qa];
-                    const PairK<P>& pb = s_pair[qb < 0 ? qa : qb];
-                    int off[EL];
-                    float ka[EL];
-#pragma unroll
-                    for (int k = 0; k < EL; ++k) {
-                        const int e = min(lane + 32 * k, WW - 1);
-                        const int dy = e / W, dx = e - dy * W;
-                        off[k] = pa.f[1][dy] * ox + pa.f[0][dx];
-                        ka[k] = (lane + 32 * k < WW) ? pa.K[1][dy] * pa.K[0][dx] : 0.0f;
-                    }
-                    float g[W][EL];
-#pragma unroll
-                    for (int dz = 0; dz < W; ++dz) {
-                        const int zo = pa.f[2][dz] * oxy;
-#pragma unroll
-                        for (int k = 0; k < EL; ++k) g[dz][k] = __ldg(G + off[k] + zo);
-                    }
-#pragma unroll
-                    for (int dz = 0; dz < W; ++dz) {
-                        float t = 0.0f;
-#pragma unroll
-                        for (int k = 0; k < EL; ++k) t = fmaf(ka[k], g[dz][k], t);
-                        acc_rec += (double)(pa.coef * pa.K[2][dz] * t);
-                    }
-                    if (qb >= 0) {
-                        float kb[EL];
-#pragma unroll
-                        for (int k = 0; k < EL; ++k) {
-                            const int e = min(lane + 32 * k, WW - 1);
-                            const int dy = e / W, dx = e - dy * W;
-                            kb[k] = (lane + 32 * k < WW) ? pb.K[1][dy] * pb.K[0][dx] : 0.0f;
-                        }
-#pragma unroll
-                        for (int dz = 0; dz < W; ++dz) {
-                            float t = 0.0f;
-#pragma unroll
-                            for (int k = 0; k < EL; ++k) t = fmaf(kb[k], g[dz][k], t);
-                            acc_rec += (double)(pb.coef * pb.K[2][dz] * t);
-                        }
-                    }
-                }
-            } else {
-            const int nrow = T.npairs * WW;
-            for (int r0 = tid; r0 < nrow; r0 += RR * NT) {
-                float gv[RR][W];
-                int qv[RR], rv[RR];
-#pragma unroll
-                for (int u = 0; u < RR; ++u) {
-                    const int rowg = min(r0 + u * NT, nrow - 1);
-                    const int q = rowg / WW, rw = rowg - q * WW;
-                    const int dz = rw / W, dy = rw - dz * W;
-                    const PairK<P>& pk = s_pair[q];
-                    const float* Grow = G + (pk.f[2][dz] * oy + pk.f[1][dy]) * ox;
-#pragma unroll
-                    for (int dx = 0; dx < W; ++dx) gv[u][dx] = __ldg(&Grow[pk.f[0][dx]]);
-                    qv[u] = q; rv[u] = rw;
-                }
-#pragma unroll
-                for (int u = 0; u < RR; ++u) {
-                    if (r0 + u * NT >= nrow) continue;
-                    const PairK<P>& pk = s_pair[qv[u]];
-                    const int dz = rv[u] / W, dy = rv[u] - dz * W;
-                    float s = 0.0f;
-#pragma unroll
-                    for (int dx = 0; dx < W; ++dx) s = fmaf(pk.K[0][dx], gv[u][dx], s);
-                    acc_rec += (double)(pk.coef * pk.K[1][dy] * pk.K[2][dz] * s);
-                }
-            }
-            }
-        }
         if (q_chk && q_blocked > 0 && (float)q_blocked >= d.quorum * (float)q_started) s_qstop = 1;
         block_sum3<NT>(acc_lj, acc_c, acc_rec, red);
         mark(5);
@@ -1467,9 +1352,28 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_mc(DevPtrs d, int mode, int ex
             if (GC) {
                 if constexpr (GC) {
                     if (sG.phase == 2) {
-                        int ops = 0;
-                        accept = p2_decide(sG, D, S, d, dlj, dc, acc_rec, dself, dqc, dslab, &ops);
+                        int ops = 0, undo = 0;
+                        accept = p2_decide(sG, D, S, d, s_npend, dlj, dc, acc_rec, dself, dqc, dslab, &ops, &undo);
                         s_gc_ops = ops;
+                        if (undo) {  // the rejected move's NH half goes back to what it was
+                            int nj = 0;
+                            for (int k = 0; k < 2; ++k) {
+                                const float4 o = sG.o_pq[k];
+                                const int gi = D.slot_off + (k ? sG.iN : sG.iP), c = cell_index(D, o.x, o.y, o.z);
+                                d.posq[gi] = o;
+                                d.type[gi] = sG.o_type[k];
+                                const int k_was = desc_class(sG.o_flags[k], sG.n_q[k]), k_is = desc_class(sG.o_flags[k], o.w);
+                                if (k_was != k_is) { cls_add(d, D, c, k_was, -1); cls_add(d, D, c, k_is, 1); }
+                                if (d.qband && o.w != sG.n_q[k]) {
+                                    if (sG.n_q[k] != 0.0f) { s_qjob[nj] = make_float4(o.x, o.y, o.z, sG.n_q[k]); s_qsgn[nj] = -1; ++nj; }
+                                    if (o.w != 0.0f) { s_qjob[nj] = o; s_qsgn[nj] = 1; ++nj; }
+                                }
+                            }
+                            s_nqjob = nj;
+                            for (int k = 0; k < 8; ++k) (&S.E)[k] = sG.o_E[k];
+                            for (int k = 0; k < 4; ++k) (&S.Q)[k] = sG.o_mom[k];
+                            s_npend = sG.o_npend;
+                        }
                     } else {
                         accept = gc_decide(sG, D, S, d, dlj, dc, acc_rec, dself, dqc, dslab);
                         s_gc_ops = accept;
@@ -1562,6 +1466,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_mc(DevPtrs d, int mode, int ex
                         d.posq[gi] = T.pn[k];
                         d.type[gi] = T.tn[k];
                         const int nc = cell_index(D, T.pn[k].x, T.pn[k].y, T.pn[k].z);
+                        const bool moved = T.po[k].x != T.pn[k].x || T.po[k].y != T.pn[k].y || T.po[k].z != T.pn[k].z;
                         if (k == 0 && T.nch == 1 && T.nprobe == 2) {
                             // displacement: the old cell's tail and the new cell's count were
                             // loaded during the parallel phase (probe 1 = new state, entry 13 = its cell)
@@ -1580,7 +1485,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_mc(DevPtrs d, int mode, int ex
                                     d.cell_pos[gi] = nn;
                                 }
                             }
-                        } else if (nc != d.cell_of[gi]) {
+                        } else if (moved && nc != d.cell_of[gi]) {
                             cell_remove(d, D, i);
                             if (!cell_insert(d, D, i, nc)) S.error = PHMC_ERR_CAPACITY;
                         }
@@ -1625,15 +1530,15 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_mc(DevPtrs d, int mode, int ex
                 const bool fwd = sG.dir > 0;
                 const int ka = fwd ? GC_NHN : GC_NHP, kb = fwd ? GC_NHP : GC_NHN;
                 const int kc = fwd ? GC_W : GC_CL, kd = fwd ? GC_CL : GC_W;
-                gc_pool_move<NT>(gc_pool(d, D, ka), gc_pool(d, D, kb), sG.n[ka], sG.n[kb], T.idx[0], &s_gc_find);
-                gc_pool_move<NT>(gc_pool(d, D, kc), gc_pool(d, D, kd), sG.n[kc], sG.n[kd], T.idx[1], &s_gc_find);
+                gc_pool_move<NT>(gc_pool(d, D, ka), gc_pool(d, D, kb), sG.n[ka], sG.n[kb], T.idx[0], sG.k[0]);
+                gc_pool_move<NT>(gc_pool(d, D, kc), gc_pool(d, D, kd), sG.n[kc], sG.n[kd], T.idx[1], sG.k[1]);
             } else if (ops >= 2) {  // phase 2's accepted move (MC/src/mc.cu:252-256, 286-287)
                 if (ops == 2) {
-                    gc_pool_move<NT>(gc_pool(d, D, GC_NHP), gc_pool(d, D, GC_NHN), sG.n[GC_NHP], sG.n[GC_NHN], sG.iP, &s_gc_find);
-                    gc_pool_move<NT>(gc_pool(d, D, GC_NHN), gc_pool(d, D, GC_NHP), sG.n[GC_NHN], sG.n[GC_NHP], sG.iN, &s_gc_find);
+                    gc_pool_move<NT>(gc_pool(d, D, GC_NHP), gc_pool(d, D, GC_NHN), sG.n[GC_NHP], sG.n[GC_NHN], sG.iP, sG.k[0]);
+                    gc_pool_move<NT>(gc_pool(d, D, GC_NHN), gc_pool(d, D, GC_NHP), sG.n[GC_NHN], sG.n[GC_NHP], sG.iN, sG.k[1]);
                 }
-                gc_pool_move<NT>(gc_pool(d, D, GC_CL), gc_pool(d, D, GC_W), sG.n[GC_CL], sG.n[GC_W], sG.jCl, &s_gc_find);
-                gc_pool_move<NT>(gc_pool(d, D, GC_W), gc_pool(d, D, GC_CL), sG.n[GC_W], sG.n[GC_CL], sG.jW, &s_gc_find);
+                gc_pool_move<NT>(gc_pool(d, D, GC_CL), gc_pool(d, D, GC_W), sG.n[GC_CL], sG.n[GC_W], sG.jCl, sG.k[2]);
+                gc_pool_move<NT>(gc_pool(d, D, GC_W), gc_pool(d, D, GC_CL), sG.n[GC_W], sG.n[GC_CL], sG.jW, sG.k[3]);
             }
             if (ops) {
                 if (tid == 0) s_gc_ops = 0;
@@ -1688,23 +1593,44 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_mc(DevPtrs d, int mode, int ex
     }
 }
 
-template <int P, int NT, int RC, int RR>
+// Raise the dynamic shared-memory cap of the engine's MC kernel instance to the
+// device maximum (minus its static shared memory), once, outside any capture.
+template <int P, int NT, int RC>
+static cudaError_t prepare_mc_t(Engine& E) {
+    int optin = 0;
+    cudaError_t e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, E.device);
+    if (e != cudaSuccess) return e;
+    auto kern = k_mc<P, NT, false, RC, true>;
+    cudaFuncAttributes fa;
+    e = cudaFuncGetAttributes(&fa, kern);
+    if (e != cudaSuccess) return e;
+    const int cap = optin - (int)fa.sharedSizeBytes;
+    if ((size_t)cap < mc_smem_bytes(P, E.pend_max, true)) return cudaErrorInvalidValue;
+    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, cap);
+}
+
+template <int P, int NT, int RC>
 static cudaError_t launch_mc_t(Engine& E, int mode, int rep, const phmc_trial* t, int n, double* dE, cudaStream_t st) {
     DevPtrs dd = E.d;
     if (E.first_stage_off) dd.sur.H = 0;  // surrogate attached but bypassed: every trial exact
-    auto kern = k_mc<P, NT, false, RC, RR, true>;
+    auto kern = k_mc<P, NT, false, RC, true>;
     size_t smem = mc_smem_bytes(P, E.pend_max, false);
     dd.sur_late_l3 = 0;
     if (dd.sur.H > 0) {
-        // three staged layers when two blocks per SM still fit, else two buffers
+        // three staged layers when the blocks an SM can hold still fit, else two buffers
         cudaFuncAttributes fa;
         cudaFuncGetAttributes(&fa, kern);
         int per_sm = 0;
         cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, E.device);
         const size_t three = mc_smem_bytes(P, E.pend_max, true);
-        const bool fits2 = 2 * (three + fa.sharedSizeBytes + 1024) <= (size_t)per_sm;
-        dd.sur_late_l3 = fits2 ? 0 : 1;
-        smem = fits2 ? three : mc_smem_bytes(P, E.pend_max, true, true);
+        const bool fits = (NT == 512 ? 1 : 2) * (three + fa.sharedSizeBytes + 1024) <= (size_t)per_sm;
+        dd.sur_late_l3 = fits ? 0 : 1;
+        smem = fits ? three : mc_smem_bytes(P, E.pend_max, true, true);
+    }
+    if (NT == 512 && E.mc512_smem < smem) {  // (the other sizes' limits are raised with the engine's shapes)
+        cudaError_t e = prepare_mc_t<P, NT, RC>(E);
+        if (e != cudaSuccess) return e;
+        E.mc512_smem = smem;
     }
     // external trials: committed ones one after the other, others as many at once as are resident
     const int grid = mode == MC_RUN ? E.R : (mode == MC_APPLY ? 1 : std::min(n, E.nsm * (512 / NT)));
@@ -1725,8 +1651,8 @@ static cudaError_t launch_mc_t(Engine& E, int mode, int rep, const phmc_trial* t
     return cudaGetLastError();
 }
 
-// One block per job of the grand-canonical phase (128 threads; no surrogate, no quorum).
-template <int P>
+// One block per job of the grand-canonical phase (no surrogate, no quorum).
+template <int P, int NT>
 static cudaError_t launch_mc_gc_t(Engine& E, int n_jobs, cudaStream_t st) {
     DevPtrs dd = E.d;
     dd.quorum = 1.0f;
@@ -1735,94 +1661,82 @@ static cudaError_t launch_mc_gc_t(Engine& E, int n_jobs, cudaStream_t st) {
     dd.log_move = nullptr;
     dd.replay = nullptr;
     dd.sur.H = 0;
+    auto kern = k_mc<P, NT, true, 4, false>;
     const size_t smem = mc_smem_bytes(P, E.pend_max, false);
     cudaFuncAttributes fa;
-    cudaError_t e = cudaFuncGetAttributes(&fa, k_mc<P, 128, true, 4, 2, false>);
+    cudaError_t e = cudaFuncGetAttributes(&fa, kern);
     if (e != cudaSuccess) return e;
     int optin = 0;
     e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, E.device);
     if (e != cudaSuccess) return e;
     if (smem + fa.sharedSizeBytes > (size_t)optin) return cudaErrorInvalidValue;
-    e = cudaFuncSetAttribute(k_mc<P, 128, true, 4, 2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    k_mc<P, 128, true, 4, 2, false><<<n_jobs, 128, smem, st>>>(dd, MC_GC, 0, nullptr, 0, nullptr, E.pend_max);
+    kern<<<n_jobs, NT, smem, st>>>(dd, MC_GC, 0, nullptr, 0, nullptr, E.pend_max);
     return cudaGetLastError();
 }
 
+// A job's evaluations are one chain: with an SM to itself a job takes a block of 512 threads (its
+// 14 to 50 windows go round 15 warps at once), with more jobs than SMs one of 128.
 cudaError_t launch_mc_gc(Engine& E, int n_jobs, cudaStream_t st) {
+    const bool wide = n_jobs <= E.nsm;
     switch (E.order) {
-        case 4: return launch_mc_gc_t<4>(E, n_jobs, st);
-        case 5: return launch_mc_gc_t<5>(E, n_jobs, st);
-        default: return launch_mc_gc_t<6>(E, n_jobs, st);
+        case 4: return wide ? launch_mc_gc_t<4, 512>(E, n_jobs, st) : launch_mc_gc_t<4, 128>(E, n_jobs, st);
+        case 5: return wide ? launch_mc_gc_t<5, 512>(E, n_jobs, st) : launch_mc_gc_t<5, 128>(E, n_jobs, st);
+        default: return wide ? launch_mc_gc_t<6, 512>(E, n_jobs, st) : launch_mc_gc_t<6, 128>(E, n_jobs, st);
     }
 }
 
-// Raise the dynamic shared-memory cap of the engine's MC kernel instance to the
-// device maximum (minus its static shared memory), once, outside any capture.
-template <int P, int NT, int RC, int RR>
-static cudaError_t prepare_mc_t(Engine& E) {
-    int optin = 0;
-    cudaError_t e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, E.device);
-    if (e != cudaSuccess) return e;
-    auto kern = k_mc<P, NT, false, RC, RR, true>;
-    cudaFuncAttributes fa;
-    e = cudaFuncGetAttributes(&fa, kern);
-    if (e != cudaSuccess) return e;
-    const int cap = optin - (int)fa.sharedSizeBytes;
-    if ((size_t)cap < mc_smem_bytes(P, E.pend_max, true)) return cudaErrorInvalidValue;
-    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, cap);
-}
-
-// The compiled (order, round width, G rows) variants: order 5 (the configurations' order)
-// has seven pair-pass shapes, orders 4 and 6 the default one.  f gets the four template
-// values as integral constants; an unsupported combination gives cudaErrorInvalidValue.
+// The compiled (order, round width) variants: order 5 (the configurations' order) has three, orders
+// 4 and 6 the default one.  The G rows field of the shapes has no bearing on the code any more (all
+// of its values read whole windows); the combinations that were refused still are.
 template <int V>
 using IC = std::integral_constant<int, V>;
 template <class F>
-static cudaError_t mc_dispatch(const Engine& E, F&& f) {
-    const bool t128 = E.threads == 128;
+static cudaError_t mc_dispatch(const Engine& E, int threads, F&& f) {
     const int rc = E.cand_round, rr = E.g_rows;
-#define MC_VARIANT(p, c, g) \
-    if (rc == c && rr == g) return t128 ? f(IC<p>{}, IC<128>{}, IC<c>{}, IC<g>{}) : f(IC<p>{}, IC<256>{}, IC<c>{}, IC<g>{});
-    switch (E.order) {
-        case 4: MC_VARIANT(4, 4, 2) break;
-        case 5:
-            MC_VARIANT(5, 4, 2) MC_VARIANT(5, 2, 2) MC_VARIANT(5, 8, 2) MC_VARIANT(5, 2, 3) MC_VARIANT(5, 2, 4)
-            MC_VARIANT(5, 2, 21) MC_VARIANT(5, 4, 21) break;
-        default: MC_VARIANT(6, 4, 2) break;
+#define MC_VARIANT(p, c)                                    \
+    {                                                       \
+        if (threads == 128) return f(IC<p>{}, IC<128>{}, IC<c>{}); \
+        if (threads == 256) return f(IC<p>{}, IC<256>{}, IC<c>{}); \
+        return f(IC<p>{}, IC<512>{}, IC<c>{});              \
     }
+    if (E.order != 5) {
+        if (rc != 4 || rr != 2) return cudaErrorInvalidValue;
+        if (E.order == 4) MC_VARIANT(4, 4)
+        MC_VARIANT(6, 4)
+    }
+    if (rc == 2) MC_VARIANT(5, 2)
+    if (rc == 4 && (rr == 2 || rr == 21)) MC_VARIANT(5, 4)
+    if (rc == 8 && rr == 2) MC_VARIANT(5, 8)
 #undef MC_VARIANT
     return cudaErrorInvalidValue;
 }
 
 cudaError_t prepare_mc(Engine& E) {
+    E.mc512_smem = 0;
     cudaError_t e = prepare_mc_run(E);
     if (e != cudaSuccess) return e;
-    return mc_dispatch(E, [&](auto p, auto nt, auto rc, auto rr) {
-        return prepare_mc_t<decltype(p)::value, decltype(nt)::value, decltype(rc)::value, decltype(rr)::value>(E);
+    return mc_dispatch(E, E.threads, [&](auto p, auto nt, auto rc) {
+        return prepare_mc_t<decltype(p)::value, decltype(nt)::value, decltype(rc)::value>(E);
     });
 }
 
 size_t mc_smem_bytes(int order, int pend_max, bool staged_surrogate, bool two_buffers) {
-    size_t st = 0, pk = 0;
-    switch (order) {
-        case 4: st = sizeof(Stencil<4>); pk = sizeof(PairK<4>); break;
-        case 5: st = sizeof(Stencil<5>); pk = sizeof(PairK<5>); break;
-        default: st = sizeof(Stencil<6>); pk = sizeof(PairK<6>); break;
-    }
-    // Monte Carlo trials carry <= 2 stencils against <= pend_max pending ones;
-    // external trials (<= NST_MAX stencils) always start with none pending
-    const size_t npairs = std::max((size_t)2 * pend_max + 3, (size_t)(NST_MAX * (NST_MAX + 1) / 2));
-    // with a surrogate attached the pair tables' space also holds its activations and staged weights
+    const size_t st = order == 4 ? mc_stencil_bytes<4>(pend_max) : (order == 5 ? mc_stencil_bytes<5>(pend_max) : mc_stencil_bytes<6>(pend_max));
+    const int tab = order == 4 ? Win<4>::TAB : (order == 5 ? Win<5>::TAB : Win<6>::TAB);
+    // with a surrogate attached the window tables' space also holds its activations and staged weights
     const size_t sur = staged_surrogate ? (size_t)(two_buffers ? SUR_SMEM2_BYTES : SUR_SMEM_BYTES) : (size_t)0;
-    return st * (pend_max + NST_MAX) + std::max(pk * npairs, sur);
+    return st + std::max(sizeof(float) * 15 * 2 * tab, sur);  // 15 warps of the largest block read windows
 }
 
 cudaError_t launch_mc(Engine& E, int mode, int rep, const phmc_trial* t, int n, double* dE, cudaStream_t st) {
     // plain Monte Carlo (no network, no harvest) runs in batches of trials (k_mc_run.cu)
     if (mode == MC_RUN && !(E.d.sur.H > 0 && !E.first_stage_off) && E.d.hv_cap == 0) return launch_mc_run(E, st);
-    return mc_dispatch(E, [&](auto p, auto nt, auto rc, auto rr) {
-        return launch_mc_t<decltype(p)::value, decltype(nt)::value, decltype(rc)::value, decltype(rr)::value>(
+    // first-stage and harvest runs: with an SM to itself a replica takes a block of 512 threads
+    const int threads = mode == MC_RUN && E.R <= E.nsm ? 512 : E.threads;
+    return mc_dispatch(E, threads, [&](auto p, auto nt, auto rc) {
+        return launch_mc_t<decltype(p)::value, decltype(nt)::value, decltype(rc)::value>(
             E, mode, rep, t, n, dE, st);
     });
 }

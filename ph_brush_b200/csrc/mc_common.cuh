@@ -4,14 +4,6 @@
 #include "common.cuh"
 #include "engine.h"
 
-template <int P>
-struct Stencil {
-    int base[3];
-    int m[3][P];   // wrapped mesh coordinates
-    float w[3][P];
-    float coef;
-};
-
 __device__ __forceinline__ float4 rand_pos(const RepDesc& D, uint32_t a, uint32_t b, uint32_t c) {
     float4 p;
     p.x = __fmul_rn(D.L[0], u24(a));
@@ -38,27 +30,6 @@ __device__ __forceinline__ int move_of(const RepDesc& D, uint32_t a0) {
     if (um < D.p_disp + D.p_titr + D.p_swap) return PHMC_MOVE_SWAP;
     return PHMC_MOVE_NONE;
 }
-
-// Axis k of the stencil of a charge at p (weights, base, wrapped mesh indices).
-template <int P>
-__device__ __forceinline__ void make_stencil_axis(Stencil<P>& s, const RepDesc& D, float4 p, int k) {
-    const float pk = (k == 0) ? p.x : (k == 1 ? p.y : p.z);
-    const float g = pk / D.L[k] * (float)D.mesh[k];
-    const float fl = floorf(g);
-    float w[P];
-    bspline_weights<P>(g - fl, w);
-    const int base = (int)fl + P / 2 - P + 1;
-    s.base[k] = base;
-#pragma unroll
-    for (int j = 0; j < P; ++j) {  // base + j lies in [-P, n + P): one correction wraps it
-        int m = base + j;
-        m += (m < 0) ? D.mesh[k] : 0;
-        m -= (m >= D.mesh[k]) ? D.mesh[k] : 0;
-        s.m[k][j] = m;
-        s.w[k][j] = w[j];
-    }
-}
-
 
 __device__ __forceinline__ int wrap1(int i, int n) { return i < 0 ? i + n : (i >= n ? i - n : i); }
 // i mod n for |i| within a few periods (descriptor cell offsets)

@@ -122,9 +122,9 @@ class Engine:
         _abi.check(self._lib.phmc_set_quorum(self._h, float(quorum)))
 
     def set_tile_shapes(self, zpass=-1, cand_round=-1, energy_block=-1, g_rows=-1, plane_pipe=-1):
-        """z pass of the rebuild (0 Stockham, k > 0 a register split), pair-pass round width,
-        full-recompute block size, G rows in flight per thread, pipelined first pass; -1 keeps
-        a field."""
+        """z pass of the rebuild (0 Stockham, k > 0 a register split), round width of the pair pass
+        (first-stage runs and external trials), threads of a full-recompute block, pipelined first
+        pass; g_rows is kept for saved tunings, without effect.  -1 keeps a field."""
         _abi.check(self._lib.phmc_set_tile_shapes(self._h, int(zpass), int(cand_round), int(g_rows),
                                                   int(energy_block), int(plane_pipe)))
 
