@@ -35,7 +35,13 @@ struct phmc_engine {
     int* h_log_move = nullptr; double* h_log_dE = nullptr; int* h_log_acc = nullptr; long long log_cap = 0;
     int* d_replay = nullptr; long long replay_n = 0;
     long long replay_cap = 0;
-    phmc_trial* d_trials = nullptr; double* d_dE = nullptr; int trials_cap = 0;
+    phmc_trial* d_trials = nullptr; double* d_dE = nullptr; int trials_cap = 0;  // d_dE: n dE, then 7 n components
+    // page-locked mirrors, one allocation with E.h_active: small copies to and from them need no
+    // staging by the driver and wait for nothing until the call's one synchronisation
+    RepState* pin_state = nullptr;      // all replicas' states at the last check_kernel_errors
+    phmc_trial* pin_trials = nullptr;   // PIN_TRIALS external trials, and 8 results each
+    double* pin_res = nullptr;
+    int* pin_cnt = nullptr;             // charged sites per replica
     std::vector<int> caps;
     // measurement
     bool profiling = false;
@@ -68,6 +74,8 @@ struct phmc_engine {
     phmc_event_fn ev_fn = nullptr;
     void* ev_user = nullptr;
 };
+
+#define PIN_TRIALS 64
 
 static void drop_graph(phmc_engine* h) {
     if (h->graph_exec) cudaGraphExecDestroy(h->graph_exec);
@@ -436,7 +444,18 @@ static int build(phmc_engine* h, int R, const phmc_system* sys, const phmc_param
     for (const RepDesc& D : E.desc) E.max_cells = std::max(E.max_cells, D.ncell[0] * D.ncell[1] * D.ncell[2]);
     DALLOC(d.partials, (size_t)R * PHMC_FULL_MAX_BPR * 8);  // any energy_block's blocks per replica
     DALLOC(E.d_active, 1);
-    CU(cudaMallocHost((void**)&E.h_active, sizeof(int)));
+    {
+        auto up = [](size_t v) { return (v + 63) / 64 * 64; };
+        const size_t o_st = 64, o_tr = o_st + up(sizeof(RepState) * R), o_rs = o_tr + up(sizeof(phmc_trial) * PIN_TRIALS),
+                     o_cn = o_rs + sizeof(double) * 8 * PIN_TRIALS;
+        unsigned char* pin = nullptr;
+        CU(cudaMallocHost((void**)&pin, o_cn + sizeof(int) * R));
+        E.h_active = reinterpret_cast<int*>(pin);
+        h->pin_state = reinterpret_cast<RepState*>(pin + o_st);
+        h->pin_trials = reinterpret_cast<phmc_trial*>(pin + o_tr);
+        h->pin_res = reinterpret_cast<double*>(pin + o_rs);
+        h->pin_cnt = reinterpret_cast<int*>(pin + o_cn);
+    }
 
     CU(cudaMemcpy(d.posq, h_posq.data(), sizeof(float4) * N, cudaMemcpyHostToDevice));
     CU(cudaMemcpy(d.type, h_type.data(), sizeof(int) * N, cudaMemcpyHostToDevice));
@@ -553,12 +572,13 @@ static int build(phmc_engine* h, int R, const phmc_system* sys, const phmc_param
     return PHMC_OK;
 }
 
+// Waits for the engine's stream; every replica's state is then in h->pin_state.
 static int check_kernel_errors(phmc_engine* h) {
     Engine& E = h->E;
+    CU(cudaMemcpyAsync(h->pin_state, E.d.state, sizeof(RepState) * E.R, cudaMemcpyDeviceToHost, E.stream));
     CU(cudaStreamSynchronize(E.stream));
     CU(cudaGetLastError());
-    std::vector<RepState> st((size_t)E.R);
-    CU(cudaMemcpy(st.data(), E.d.state, sizeof(RepState) * E.R, cudaMemcpyDeviceToHost));
+    const RepState* st = h->pin_state;
     for (int r = 0; r < E.R; ++r)
         if (st[r].error) {
             char b[160];
@@ -700,9 +720,7 @@ extern "C" int phmc_energy(phmc_engine* h, phmc_energy_components* out) {
     CU(cudaSetDevice(E.device));
     int s = full_recompute(h);
     if (s) return s;
-    std::vector<RepState> st((size_t)E.R);
-    CU(cudaMemcpy(st.data(), E.d.state, sizeof(RepState) * E.R, cudaMemcpyDeviceToHost));
-    for (int r = 0; r < E.R; ++r) fill_components(st[r], &out[r]);
+    for (int r = 0; r < E.R; ++r) fill_components(h->pin_state[r], &out[r]);
     return PHMC_OK;
 }
 
@@ -727,9 +745,31 @@ static int ensure_trial_buffers(phmc_engine* h, int n) {
     if (n <= h->trials_cap) return PHMC_OK;
     if (h->d_trials) { cudaFree(h->d_trials); cudaFree(h->d_dE); h->d_trials = nullptr; h->d_dE = nullptr; }
     CU(cudaMalloc((void**)&h->d_trials, sizeof(phmc_trial) * n));
-    CU(cudaMalloc((void**)&h->d_dE, sizeof(double) * n));
+    CU(cudaMalloc((void**)&h->d_dE, sizeof(double) * 8 * (size_t)n));
     h->trials_cap = n;
     return PHMC_OK;
+}
+
+// Judge n external trials: their dE (res[0 .. n)) and, with comps, 7 components each after them.
+static int judge_trials(phmc_engine* h, int rep, const phmc_trial* trials, int n, bool comps, double* res) {
+    int s = check_trials(h, rep, trials, n);
+    if (s) return s;
+    Engine& E = h->E;
+    CU(cudaSetDevice(E.device));
+    s = ensure_trial_buffers(h, n);
+    if (s) return s;
+    const bool pin = n <= PIN_TRIALS;
+    const size_t bytes = sizeof(double) * (comps ? 8 : 1) * (size_t)n;
+    if (pin) std::memcpy(h->pin_trials, trials, sizeof(phmc_trial) * n);
+    CU(cudaMemcpyAsync(h->d_trials, pin ? h->pin_trials : trials, sizeof(phmc_trial) * n, cudaMemcpyHostToDevice, E.stream));
+    E.d.ext_comp = comps ? h->d_dE + n : nullptr;
+    const cudaError_t e = launch_mc(E, MC_EVAL, rep, h->d_trials, n, h->d_dE, E.stream);
+    E.d.ext_comp = nullptr;
+    if (e != cudaSuccess) return fail(PHMC_ERR_CUDA, std::string("external trials: ") + cudaGetErrorString(e));
+    CU(cudaMemcpyAsync(pin ? h->pin_res : res, h->d_dE, bytes, cudaMemcpyDeviceToHost, E.stream));
+    s = check_kernel_errors(h);
+    if (pin) std::memcpy(res, h->pin_res, bytes);
+    return s;
 }
 
 static int flush_dirty(phmc_engine* h) {
@@ -744,16 +784,7 @@ static int flush_dirty(phmc_engine* h) {
 extern "C" int phmc_delta_energy(phmc_engine* h, int rep, const phmc_trial* trials, int n, double* dE) {
     if (!h || (n > 0 && (!trials || !dE))) return fail(PHMC_ERR_ARG, "null argument");
     if (n == 0) return PHMC_OK;
-    int s = check_trials(h, rep, trials, n);
-    if (s) return s;
-    Engine& E = h->E;
-    CU(cudaSetDevice(E.device));
-    s = ensure_trial_buffers(h, n);
-    if (s) return s;
-    CU(cudaMemcpyAsync(h->d_trials, trials, sizeof(phmc_trial) * n, cudaMemcpyHostToDevice, E.stream));
-    CU(launch_mc(E, MC_EVAL, rep, h->d_trials, n, h->d_dE, E.stream));
-    CU(cudaMemcpyAsync(dE, h->d_dE, sizeof(double) * n, cudaMemcpyDeviceToHost, E.stream));
-    return check_kernel_errors(h);
+    return judge_trials(h, rep, trials, n, false, dE);
 }
 
 extern "C" int phmc_commit(phmc_engine* h, int rep, const phmc_trial* trial) {
@@ -764,7 +795,8 @@ extern "C" int phmc_commit(phmc_engine* h, int rep, const phmc_trial* trial) {
     CU(cudaSetDevice(E.device));
     s = ensure_trial_buffers(h, 1);
     if (s) return s;
-    CU(cudaMemcpyAsync(h->d_trials, trial, sizeof(phmc_trial), cudaMemcpyHostToDevice, E.stream));
+    h->pin_trials[0] = *trial;
+    CU(cudaMemcpyAsync(h->d_trials, h->pin_trials, sizeof(phmc_trial), cudaMemcpyHostToDevice, E.stream));
     CU(launch_mc(E, MC_APPLY, rep, h->d_trials, 1, h->d_dE, E.stream));
     s = flush_dirty(h);
     if (s) return s;
@@ -854,27 +886,20 @@ __global__ void k_count_charged(DevPtrs d, int* __restrict__ out) {
     }
 }
 
-static int collect_stats(phmc_engine* h, phmc_run_stats* stats) {
+// Statistics of the run from the states and charged-site counts that the last check brought back.
+static void collect_stats(phmc_engine* h, phmc_run_stats* stats) {
     Engine& E = h->E;
-    std::vector<RepState> st((size_t)E.R);
-    CU(cudaMemcpy(st.data(), E.d.state, sizeof(RepState) * E.R, cudaMemcpyDeviceToHost));
     for (int r = 0; r < E.R; ++r) {
+        const RepState& st = h->pin_state[r];
         phmc_run_stats& o = stats[r];
         std::memset(&o, 0, sizeof o);
-        for (int k = 0; k < 3; ++k) { o.attempted[k] = st[r].att[k]; o.accepted[k] = st[r].acc[k]; }
-        o.flushes = st[r].flushes;
+        for (int k = 0; k < 3; ++k) { o.attempted[k] = st.att[k]; o.accepted[k] = st.acc[k]; }
+        o.flushes = st.flushes;
         o.n_titratable = E.desc[r].n_titr;
-        o.n_cations = st[r].n_cation; o.n_anions = st[r].n_anion;
-        o.energy = st[r].E; o.energy_drift = st[r].drift;
+        o.n_charged_sites = h->pin_cnt[r];
+        o.n_cations = st.n_cation; o.n_anions = st.n_anion;
+        o.energy = st.E; o.energy_drift = st.drift;
     }
-    // protonated sites: titratable sites with q != 0, counted on the device
-    if (!h->d_charged) CU(cudaMalloc((void**)&h->d_charged, sizeof(int) * E.R));
-    k_count_charged<<<E.R, 1024, 0, E.stream>>>(E.d, h->d_charged);
-    std::vector<int> cnt((size_t)E.R);
-    CU(cudaMemcpyAsync(cnt.data(), h->d_charged, sizeof(int) * E.R, cudaMemcpyDeviceToHost, E.stream));
-    CU(cudaStreamSynchronize(E.stream));
-    for (int r = 0; r < E.R; ++r) stats[r].n_charged_sites = cnt[(size_t)r];
-    return PHMC_OK;
 }
 
 // Run the trial/rebuild loop (internal; also used by the timed entry points).
@@ -1042,6 +1067,11 @@ extern "C" int phmc_run(phmc_engine* h, int64_t n_trials, phmc_run_stats* stats)
     CU(cudaSetDevice(E.device));
     int s = phmc_run_loop(h, n_trials, 4);
     if (s) return s;
+    if (stats) {  // protonated sites: titratable sites with q != 0, counted on the device
+        if (!h->d_charged) CU(cudaMalloc((void**)&h->d_charged, sizeof(int) * E.R));
+        k_count_charged<<<E.R, 1024, 0, E.stream>>>(E.d, h->d_charged);
+        CU(cudaMemcpyAsync(h->pin_cnt, h->d_charged, sizeof(int) * E.R, cudaMemcpyDeviceToHost, E.stream));
+    }
     s = check_kernel_errors(h);
     if (s) return s;
     if (h->h_log_move && E.d.log_move) {
@@ -1054,7 +1084,7 @@ extern "C" int phmc_run(phmc_engine* h, int64_t n_trials, phmc_run_stats* stats)
             CU(cudaMemcpy(h->h_da_dEs, E.d.log_dEs, sizeof(double) * n, cudaMemcpyDeviceToHost));
         }
     }
-    if (stats) return collect_stats(h, stats);
+    if (stats) collect_stats(h, stats);
     return PHMC_OK;
 }
 
@@ -2054,31 +2084,15 @@ extern "C" int phmc_autotune(phmc_engine* h, int64_t trials, phmc_tuning* result
 extern "C" int phmc_delta_energy_components(phmc_engine* h, int rep, const phmc_trial* trials, int n,
                                             phmc_energy_components* out) {
     if (!h || (n > 0 && (!trials || !out))) return fail(PHMC_ERR_ARG, "null argument");
-    if (n == 0) return PHMC_OK;
-    int s = check_trials(h, rep, trials, n);
-    if (s) return s;
-    Engine& E = h->E;
-    CU(cudaSetDevice(E.device));
-    s = ensure_trial_buffers(h, n);
-    if (s) return s;
-    double* d_c = nullptr;
-    CU(cudaMalloc((void**)&d_c, sizeof(double) * 7 * (size_t)n));
-    cudaError_t e = cudaMemcpyAsync(h->d_trials, trials, sizeof(phmc_trial) * n, cudaMemcpyHostToDevice, E.stream);
-    E.d.ext_comp = d_c;
-    if (e == cudaSuccess) e = launch_mc(E, MC_EVAL, rep, h->d_trials, n, h->d_dE, E.stream);
-    E.d.ext_comp = nullptr;
-    std::vector<double> hc((size_t)7 * n), dE((size_t)n);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(hc.data(), d_c, sizeof(double) * 7 * n, cudaMemcpyDeviceToHost, E.stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(dE.data(), h->d_dE, sizeof(double) * n, cudaMemcpyDeviceToHost, E.stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(E.stream);
-    cudaFree(d_c);
-    if (e != cudaSuccess) return fail(PHMC_ERR_CUDA, std::string("delta_energy_components: ") + cudaGetErrorString(e));
-    for (int k = 0; k < n; ++k) {
-        const double* c = hc.data() + 7 * k;
+    if (n <= 0) return PHMC_OK;
+    std::vector<double> res((size_t)8 * n);
+    const int s = judge_trials(h, rep, trials, n, true, res.data());
+    for (int k = 0; k < n && (s == PHMC_OK || s == PHMC_ERR_CAPACITY); ++k) {
+        const double* c = res.data() + n + 7 * (size_t)k;
         out[k].lj = c[0]; out[k].fene = c[1]; out[k].coul_real = c[2]; out[k].coul_recip = c[3];
-        out[k].self = c[4]; out[k].qcorr = c[5]; out[k].slab = c[6]; out[k].total = dE[(size_t)k];
+        out[k].self = c[4]; out[k].qcorr = c[5]; out[k].slab = c[6]; out[k].total = res[(size_t)k];
     }
-    return check_kernel_errors(h);
+    return s;
 }
 
 // ---------------------------------------------------------------------------

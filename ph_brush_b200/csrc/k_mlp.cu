@@ -361,6 +361,7 @@ struct phmc_surrogate {
     uint2* packed[3] = {nullptr, nullptr, nullptr};  // fragment-packed hidden layers
     bool packed_ok = false;
     long cap = 0;                       // row capacity of the activation buffers
+    unsigned char* act = nullptr;       // their allocation
     __nv_bfloat16* X = nullptr;
     float* Z[3] = {nullptr, nullptr, nullptr};
     __nv_bfloat16* Hb[3] = {nullptr, nullptr, nullptr};
@@ -372,8 +373,14 @@ struct phmc_surrogate {
     float* d_scale = nullptr;
     float* split = nullptr;             // split-K partial products (GEMM_MAX_SPLITS x max(n_in, H) x H)
     int adam_t = 0;
+    unsigned char* in = nullptr;        // staging of a call's inputs (stage_inputs), kept up to SUR_KEEP bytes
+    size_t in_cap = 0;
     std::vector<void*> allocs;
 };
+
+// A call's input staging is kept with the network up to this size (a training batch of 4096 samples
+// takes 5 MB; allocating and freeing it took two thirds of a gradient's time), larger ones are freed.
+#define SUR_KEEP ((size_t)64 << 20)
 
 #define MCU(x)                                                                                     \
     do {                                                                                           \
@@ -394,6 +401,25 @@ static void free_t(phmc_surrogate* h, void* p) {
     h->allocs.erase(std::remove(h->allocs.begin(), h->allocs.end(), p), h->allocs.end());
 }
 
+// Device room for a call's inputs, `bytes` in all.
+static int stage_inputs(phmc_surrogate* h, size_t bytes) {
+    if (bytes <= h->in_cap) return PHMC_OK;
+    free_t(h, h->in);
+    h->in = nullptr;
+    h->in_cap = 0;
+    const size_t want = std::max(bytes, (size_t)1 << 20);
+    const int s = malloc_t(h, &h->in, want);
+    if (s == PHMC_OK) h->in_cap = want;
+    return s;
+}
+static void release_inputs(phmc_surrogate* h) {
+    if (h->in_cap <= SUR_KEEP) return;
+    free_t(h, h->in);
+    h->in = nullptr;
+    h->in_cap = 0;
+}
+static size_t up256(size_t v) { return (v + 255) / 256 * 256; }
+
 // parameter layout (FP32 master, flat): W1[nin*H], b1[H], W2[H*H], b2[H], W3[H*H], b3[H], w4[H], b4[1];
 // W[k*H + j] connects input k to output j
 static void layout(int nin, int H, int off[8], int* total) {
@@ -409,22 +435,28 @@ static void layout(int nin, int H, int off[8], int* total) {
     *total = o;
 }
 
+// Activation buffers of n rows, one allocation for all of them (twelve made a first call wait).
 static int ensure_rows(phmc_surrogate* h, long n) {
     if (n <= h->cap) return PHMC_OK;
-    void* old[] = {h->X, h->Z[0], h->Z[1], h->Z[2], h->Hb[0], h->Hb[1], h->Hb[2], h->dZ[0], h->dZ[1], h->dZ[2], h->y, h->dy};
-    for (void* p : old) free_t(h, p);
+    free_t(h, h->act);
+    h->act = nullptr;
     h->cap = 0;
-    const long c = std::max(n, 4096L);
+    const size_t c = (size_t)std::max(n, 4096L);
+    const size_t bx = up256(c * h->nin * sizeof(__nv_bfloat16)), bz = up256(c * h->H * sizeof(float)),
+                 bh = up256(c * h->H * sizeof(__nv_bfloat16)), by = up256(c * sizeof(float));
     int s;
-    if ((s = malloc_t(h, &h->X, (size_t)c * h->nin))) return s;
+    if ((s = malloc_t(h, &h->act, bx + 3 * (bz + 2 * bh) + 2 * by))) return s;
+    unsigned char* p = h->act;
+    auto take = [&](size_t bytes) { unsigned char* q = p; p += bytes; return q; };
+    h->X = reinterpret_cast<__nv_bfloat16*>(take(bx));
     for (int l = 0; l < 3; ++l) {
-        if ((s = malloc_t(h, &h->Z[l], (size_t)c * h->H))) return s;
-        if ((s = malloc_t(h, &h->Hb[l], (size_t)c * h->H))) return s;
-        if ((s = malloc_t(h, &h->dZ[l], (size_t)c * h->H))) return s;
+        h->Z[l] = reinterpret_cast<float*>(take(bz));
+        h->Hb[l] = reinterpret_cast<__nv_bfloat16*>(take(bh));
+        h->dZ[l] = reinterpret_cast<__nv_bfloat16*>(take(bh));
     }
-    if ((s = malloc_t(h, &h->y, c))) return s;
-    if ((s = malloc_t(h, &h->dy, c))) return s;
-    h->cap = c;
+    h->y = reinterpret_cast<float*>(take(by));
+    h->dy = reinterpret_cast<float*>(take(by));
+    h->cap = (long)c;
     return PHMC_OK;
 }
 
@@ -558,13 +590,13 @@ extern "C" int phmc_surrogate_predict(phmc_surrogate* h, const float* x, int n, 
     if (n == 0) return PHMC_OK;
     int s = ensure_rows(h, n);
     if (s) return s;
-    float* dx = nullptr;
-    MCU(cudaMalloc(&dx, sizeof(float) * (size_t)n * h->nin));
+    if ((s = stage_inputs(h, sizeof(float) * (size_t)n * h->nin))) return s;
+    float* dx = reinterpret_cast<float*>(h->in);
     cudaMemcpy(dx, x, sizeof(float) * (size_t)n * h->nin, cudaMemcpyHostToDevice);
     k_normalize<<<(int)(((long)n * h->nin + 255) / 256), 256>>>(dx, nullptr, n, h->nin, h->mu, h->sd, h->X);
     forward_rows(h, n, h->scale, 0.0f, 0);
     cudaError_t e = cudaMemcpy(y, h->y, sizeof(float) * n, cudaMemcpyDeviceToHost);
-    cudaFree(dx);
+    release_inputs(h);
     if (e != cudaSuccess) { phmc_set_error(PHMC_ERR_CUDA, cudaGetErrorString(e)); return PHMC_ERR_CUDA; }
     return gemm_status();
 }
@@ -579,10 +611,9 @@ extern "C" int phmc_surrogate_gradient(phmc_surrogate* h, const float* x, const 
     const long rows = (long)n * SUR_ROWS;
     int s = ensure_rows(h, rows);
     if (s) return s;
-    float *dx = nullptr, *ds = nullptr, *dt = nullptr;
-    MCU(cudaMalloc(&dx, sizeof(float) * (size_t)rows * h->nin));
-    MCU(cudaMalloc(&ds, sizeof(float) * (size_t)rows));
-    MCU(cudaMalloc(&dt, sizeof(float) * n));
+    const size_t bx = up256(sizeof(float) * (size_t)rows * h->nin), bs = up256(sizeof(float) * (size_t)rows);
+    if ((s = stage_inputs(h, bx + bs + sizeof(float) * n))) return s;
+    float *dx = reinterpret_cast<float*>(h->in), *ds = reinterpret_cast<float*>(h->in + bx), *dt = reinterpret_cast<float*>(h->in + bx + bs);
     cudaMemcpy(dx, x, sizeof(float) * (size_t)rows * h->nin, cudaMemcpyHostToDevice);
     cudaMemcpy(ds, sign, sizeof(float) * rows, cudaMemcpyHostToDevice);
     cudaMemcpy(dt, t, sizeof(float) * n, cudaMemcpyHostToDevice);
@@ -592,7 +623,7 @@ extern "C" int phmc_surrogate_gradient(phmc_surrogate* h, const float* x, const 
     backward_rows(h, ds, dt, nullptr, n, clip, 0);
     cudaError_t e = cudaMemcpy(grad, h->grad, sizeof(float) * h->nparam, cudaMemcpyDeviceToHost);
     if (e == cudaSuccess) e = cudaMemcpy(loss, h->loss, sizeof(double), cudaMemcpyDeviceToHost);
-    cudaFree(dx); cudaFree(ds); cudaFree(dt);
+    release_inputs(h);
     if (e != cudaSuccess) { phmc_set_error(PHMC_ERR_CUDA, cudaGetErrorString(e)); return PHMC_ERR_CUDA; }
     return gemm_status();
 }
@@ -652,15 +683,15 @@ extern "C" int phmc_surrogate_train(phmc_surrogate* h, const float* x, const flo
                                     int batch, float lr, float clip, uint64_t seed, int rescale, double* last_loss) {
     if (!h || !x || !sign || !t || n < 1) { phmc_set_error(PHMC_ERR_ARG, "phmc_surrogate_train: bad argument"); return PHMC_ERR_ARG; }
     const size_t rows = (size_t)n * SUR_ROWS;
-    float *dx = nullptr, *ds = nullptr, *dt = nullptr;
-    MCU(cudaMalloc(&dx, sizeof(float) * rows * h->nin));
-    MCU(cudaMalloc(&ds, sizeof(float) * rows));
-    MCU(cudaMalloc(&dt, sizeof(float) * n));
+    const size_t bx = up256(sizeof(float) * rows * h->nin), bs = up256(sizeof(float) * rows);
+    const int s0 = stage_inputs(h, bx + bs + sizeof(float) * n);
+    if (s0) return s0;
+    float *dx = reinterpret_cast<float*>(h->in), *ds = reinterpret_cast<float*>(h->in + bx), *dt = reinterpret_cast<float*>(h->in + bx + bs);
     cudaMemcpy(dx, x, sizeof(float) * rows * h->nin, cudaMemcpyHostToDevice);
     cudaMemcpy(ds, sign, sizeof(float) * rows, cudaMemcpyHostToDevice);
     cudaMemcpy(dt, t, sizeof(float) * n, cudaMemcpyHostToDevice);
     const int s = sur_train_device(h, dx, ds, dt, n, epochs, batch, lr, clip, seed, rescale, last_loss);
-    cudaFree(dx); cudaFree(ds); cudaFree(dt);
+    release_inputs(h);
     return s;
 }
 

@@ -4,10 +4,24 @@ Thin: every call goes through libphmc.so; arrays are converted to the ABI's
 plain pointers.  Errors raise PhmcError with the library's message.
 """
 import ctypes as C
+import operator
+import struct
 
 import numpy as np
 
 from . import _abi
+
+# one phmc_trial with one or two changes, packed as the ABI lays it out
+_FIELDS = operator.itemgetter("index", "x", "y", "z", "q", "type")
+_TRIAL = (None, struct.Struct("iiiffffi28x"), struct.Struct("iiiffffiiiffffi"))
+_COMPONENTS = tuple(k for k, _ in _abi.EnergyComponents._fields_)
+assert all(s is None or s.size == C.sizeof(_abi.Trial) for s in _TRIAL)
+
+
+def _components(out):
+    """The dicts of an array of energy components."""
+    rows = np.frombuffer(out, np.float64).reshape(-1, len(_COMPONENTS)).tolist()
+    return [dict(zip(_COMPONENTS, r)) for r in rows]
 
 
 class Engine:
@@ -50,7 +64,7 @@ class Engine:
     def energy(self):
         out = (_abi.EnergyComponents * self.R)()
         _abi.check(self._lib.phmc_energy(self._h, out))
-        return [o.asdict() for o in out]
+        return _components(out)
 
     @staticmethod
     def make_trial(changes):
@@ -63,19 +77,41 @@ class Engine:
             c.type = int(ch["type"])
         return t
 
+    @classmethod
+    def _trials(cls, trials):
+        """A ctypes array of the trials; what does not pack as it stands (a number of another type)
+        goes through make_trial's conversions."""
+        arr = (_abi.Trial * len(trials))()
+        size, off = C.sizeof(_abi.Trial), 0
+        for k, t in enumerate(trials):
+            try:
+                if len(t) == 1:
+                    i, x, y, z, q, ty = _FIELDS(t[0])
+                    _TRIAL[1].pack_into(arr, off, 1, i, t[0].get("present", 1), x, y, z, q, ty)
+                else:
+                    a, b = t
+                    i, x, y, z, q, ty = _FIELDS(a)
+                    j, u, v, w, p, tz = _FIELDS(b)
+                    _TRIAL[2].pack_into(arr, off, 2, i, a.get("present", 1), x, y, z, q, ty,
+                                        j, b.get("present", 1), u, v, w, p, tz)
+            except (struct.error, OverflowError, TypeError, ValueError, AttributeError):
+                arr[k] = cls.make_trial(t)
+            off += size
+        return arr
+
     def delta_energy(self, trials, replica=0):
         n = len(trials)
-        arr = (_abi.Trial * n)(*[self.make_trial(t) for t in trials])
+        arr = self._trials(trials)
         dE = np.zeros(n, np.float64)
         _abi.check(self._lib.phmc_delta_energy(self._h, replica, arr, n, _abi.dptr(dE)))
         return dE
 
     def delta_energy_components(self, trials, replica=0):
         n = len(trials)
-        arr = (_abi.Trial * n)(*[self.make_trial(t) for t in trials])
+        arr = self._trials(trials)
         out = (_abi.EnergyComponents * n)()
         _abi.check(self._lib.phmc_delta_energy_components(self._h, replica, arr, n, out))
-        return [o.asdict() for o in out]
+        return _components(out)
 
     def commit(self, changes, replica=0):
         t = self.make_trial(changes)
