@@ -229,39 +229,74 @@ __global__ void k_out_backward(const float* __restrict__ dy, const float* __rest
     dZ[e] = __float2bfloat16(dy[i] * __bfloat162float(__ushort_as_bfloat16(w4[k])) * gelu_grad(Z[e]));
 }
 
-// dw4[k] = sum_i dy_i h_ik, db4 = sum_i dy_i (block K handles the bias)
-__global__ void k_out_wgrad(const float* __restrict__ dy, const __nv_bfloat16* __restrict__ H, long n, int K,
-                            float* __restrict__ gw, float* __restrict__ gb) {
-    const int k = blockIdx.x;
-    float s = 0.0f;
-    for (long i = threadIdx.x; i < n; i += blockDim.x) s += dy[i] * (k < K ? __bfloat162float(H[i * K + k]) : 1.0f);
-    __shared__ float red[32];
+// Column sums over n rows, one job per blockIdx.y: the bias gradients of the three hidden layers
+// (job l: sum_i dZ_l[i][j]), and (job 3) dw4[j] = sum_i dy_i H3[i][j] with db4 = sum_i dy_i.  A block
+// sums a range of rows, lanes on consecutive column pairs; a job's last block adds the blocks' sums
+// in block order.  (A block per column read its column with a stride of a row: 45 us for the four at
+// 16384 x 128, 14 us here.)
+#define CSUM_NB 128
+__global__ void __launch_bounds__(256) k_colsums(const __nv_bfloat16* __restrict__ Z0, const __nv_bfloat16* __restrict__ Z1,
+                                                 const __nv_bfloat16* __restrict__ Z2, const __nv_bfloat16* __restrict__ H3,
+                                                 const float* __restrict__ dy, long n, int H, float* __restrict__ part,
+                                                 unsigned* __restrict__ ticket, float* __restrict__ g0, float* __restrict__ g1,
+                                                 float* __restrict__ g2, float* __restrict__ gw, float* __restrict__ gb) {
+    __shared__ float2 s_sum[256];
+    __shared__ float s_dy[256];
+    __shared__ int s_last;
+    const int job = blockIdx.y, hp = H / 2, ng = 256 / hp, tid = threadIdx.x;
+    const int g = tid / hp, cp = tid - g * hp;
+    const __nv_bfloat162* X = reinterpret_cast<const __nv_bfloat162*>(job == 0 ? Z0 : (job == 1 ? Z1 : (job == 2 ? Z2 : H3)));
+    const long per = (n + CSUM_NB - 1) / CSUM_NB, r0 = blockIdx.x * per, r1 = min(n, r0 + per);
+    float2 s = make_float2(0.0f, 0.0f);
+    float sd = 0.0f;
+    if (g < ng) {
+        constexpr int U = 8;  // rows in flight per thread
+        for (long r = r0 + g; r < r1; r += U * ng) {
+            __nv_bfloat162 x[U];
+            float w[U];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        float tot = 0.0f;
-        for (int w = 0; w < (int)blockDim.x / 32; ++w) tot += red[w];
-        if (k < K) gw[k] = tot; else *gb = tot;
-    }
-}
-
-// column sums of a bf16 matrix (bias gradients)
-__global__ void k_colsum(const __nv_bfloat16* __restrict__ X, long n, int N, float* __restrict__ out) {
-    const int j = blockIdx.x;
-    float s = 0.0f;
-    for (long i = threadIdx.x; i < n; i += blockDim.x) s += __bfloat162float(X[i * N + j]);
-    __shared__ float red[32];
+            for (int u = 0; u < U; ++u) {
+                const long rr = r + u * ng;
+                x[u] = rr < r1 ? X[rr * hp + cp] : __floats2bfloat162_rn(0.0f, 0.0f);
+                w[u] = rr < r1 ? (job == 3 ? dy[rr] : 1.0f) : 0.0f;
+            }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        float tot = 0.0f;
-        for (int w = 0; w < (int)blockDim.x / 32; ++w) tot += red[w];
-        out[j] = tot;
+            for (int u = 0; u < U; ++u) {
+                const float2 v = __bfloat1622float2(x[u]);
+                s.x += w[u] * v.x;
+                s.y += w[u] * v.y;
+                sd += w[u];
+            }
+        }
     }
+    s_sum[tid] = s;
+    s_dy[tid] = sd;
+    __syncthreads();
+    float* p = part + ((size_t)job * CSUM_NB + blockIdx.x) * (SUR_HMAX + 1);
+    if (tid < hp) {
+        for (int k = 1; k < ng; ++k) { s.x += s_sum[k * hp + tid].x; s.y += s_sum[k * hp + tid].y; }
+        p[2 * tid] = s.x;
+        p[2 * tid + 1] = s.y;
+        if (tid == 0) {
+            for (int k = 1; k < ng; ++k) sd += s_dy[k * hp];
+            p[H] = sd;
+        }
+    }
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) s_last = atomicAdd(&ticket[job], 1u) == CSUM_NB - 1;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    const float* q = part + (size_t)job * CSUM_NB * (SUR_HMAX + 1);
+    if (tid <= H) {
+        float t = 0.0f;
+#pragma unroll 16
+        for (int k = 0; k < CSUM_NB; ++k) t += __ldcg(q + (size_t)k * (SUR_HMAX + 1) + tid);  // (past this SM's L1)
+        if (tid < H) (job == 0 ? g0 : (job == 1 ? g1 : (job == 2 ? g2 : gw)))[tid] = t;
+        else if (job == 3) *gb = t;
+    }
+    if (tid == 0) ticket[job] = 0u;
 }
 
 // Adam (Kingma & Ba 2015) on the FP32 master copy, then the BF16 working copy.
@@ -372,6 +407,8 @@ struct phmc_surrogate {
     float *adam_m = nullptr, *adam_v = nullptr;
     float* d_scale = nullptr;
     float* split = nullptr;             // split-K partial products (GEMM_MAX_SPLITS x max(n_in, H) x H)
+    float* csum = nullptr;              // partial column sums of k_colsums, and its jobs' tickets (zero between launches)
+    unsigned* ticket = nullptr;
     int adam_t = 0;
     unsigned char* in = nullptr;        // staging of a call's inputs (stage_inputs), kept up to SUR_KEEP bytes
     size_t in_cap = 0;
@@ -488,10 +525,13 @@ extern "C" int phmc_surrogate_create(int n_in, int hidden, uint64_t seed, phmc_s
         (s = malloc_t(h, &h->mu, n_in)) || (s = malloc_t(h, &h->sd, n_in)) || (s = malloc_t(h, &h->loss, 1)) ||
         (s = malloc_t(h, &h->d_scale, 1)) || (s = malloc_t(h, &h->packed[0], (size_t)nk1 * hidden / 4)) ||
         (s = malloc_t(h, &h->split, (size_t)GEMM_MAX_SPLITS * std::max(n_in, hidden) * hidden)) ||
+        (s = malloc_t(h, &h->csum, (size_t)4 * CSUM_NB * (SUR_HMAX + 1) + 4)) ||
         (s = malloc_t(h, &h->packed[1], (size_t)hidden * hidden / 4)) || (s = malloc_t(h, &h->packed[2], (size_t)hidden * hidden / 4))) {
         phmc_surrogate_destroy(h);
         return s;
     }
+    h->ticket = reinterpret_cast<unsigned*>(h->csum + (size_t)4 * CSUM_NB * (SUR_HMAX + 1));
+    cudaMemset(h->ticket, 0, 4 * sizeof(unsigned));
     std::vector<float> mu((size_t)n_in, 0.0f), sd((size_t)n_in, 1.0f);
     cudaMemcpy(h->p, p.data(), sizeof(float) * p.size(), cudaMemcpyHostToDevice);
     cudaMemcpy(h->mu, mu.data(), sizeof(float) * mu.size(), cudaMemcpyHostToDevice);
@@ -534,19 +574,18 @@ static void backward_rows(phmc_surrogate* h, const float* d_sign, const float* d
     const int* off = h->off;
     const long n = (long)B * SUR_ROWS;
     k_loss<<<(B + 255) / 256, 256, 0, st>>>(h->y, d_sign, d_t, d_idx, B, h->scale, clip, h->dy, h->loss);
-    k_out_wgrad<<<H + 1, 256, 0, st>>>(h->dy, h->Hb[2], n, H, h->grad + off[6], h->grad + off[7]);
     k_out_backward<<<(int)((n * H + 255) / 256), 256, 0, st>>>(h->dy, h->Z[2], n, H, reinterpret_cast<const uint16_t*>(W + off[6]), h->dZ[2]);
     // layer 3: dW3 = H2^T dZ3, db3 = colsum dZ3, dZ2 = (dZ3 W3^T) * gelu'(Z2)
     gemm(H, H, (int)n, h->Hb[1], 1, H, h->dZ[2], H, 1, EPI_STORE, h->grad + off[4], nullptr, nullptr, nullptr, st, h->split);
-    k_colsum<<<H, 256, 0, st>>>(h->dZ[2], n, H, h->grad + off[5]);
     gemm((int)n, H, H, h->dZ[2], H, 1, W + off[4], 1, H, EPI_GELU_GRAD, nullptr, nullptr, h->Z[1], h->dZ[1], st);
     // layer 2
     gemm(H, H, (int)n, h->Hb[0], 1, H, h->dZ[1], H, 1, EPI_STORE, h->grad + off[2], nullptr, nullptr, nullptr, st, h->split);
-    k_colsum<<<H, 256, 0, st>>>(h->dZ[1], n, H, h->grad + off[3]);
     gemm((int)n, H, H, h->dZ[1], H, 1, W + off[2], 1, H, EPI_GELU_GRAD, nullptr, nullptr, h->Z[0], h->dZ[0], st);
     // layer 1
     gemm(nin, H, (int)n, h->X, 1, nin, h->dZ[0], H, 1, EPI_STORE, h->grad + off[0], nullptr, nullptr, nullptr, st, h->split);
-    k_colsum<<<H, 256, 0, st>>>(h->dZ[0], n, H, h->grad + off[1]);
+    k_colsums<<<dim3(CSUM_NB, 4), 256, 0, st>>>(h->dZ[0], h->dZ[1], h->dZ[2], h->Hb[2], h->dy, n, H, h->csum, h->ticket,
+                                                h->grad + off[1], h->grad + off[3], h->grad + off[5], h->grad + off[6],
+                                                h->grad + off[7]);
 }
 
 extern "C" int phmc_surrogate_set_scaling(phmc_surrogate* h, const float* mu, const float* sd, float scale) {
