@@ -90,6 +90,8 @@ static int flush_dirty(phmc_engine* h);
 // shared memory the kernel needs.  The caller raises the kernel's shared-memory cap.
 static void select_zpass(Engine& E, int id) {
     E.zreg = id;
+    E.zband = id != 0;
+    for (const RepDesc& D : E.desc) E.zband = E.zband && zband_fits(id, D.mesh[2], D.zb_lo, D.zb_n);
     if (id) { E.d_zjobs = E.d_zj_reg; E.n_zjobs = E.n_zj_reg; E.d_zjob_off = E.d_zoff_reg; E.zpass_smem = E.zpass_smem_reg; }
     else { E.d_zjobs = E.d_zj_stk; E.n_zjobs = E.n_zj_stk; E.d_zjob_off = E.d_zoff_stk; E.zpass_smem = E.zpass_smem_stk; }
 }

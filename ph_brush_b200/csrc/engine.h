@@ -50,6 +50,7 @@ struct Engine {
     long long total_qband = 0;   // points of the wall bands' fixed-point charge meshes
     int zreg = 0;                // active register z-pass variant for the shared nz (0: shared-memory z pass)
     int zreg_default = 0;        // the default register variant of that nz (0: none; the Stockham pass only)
+    bool zband = false;          // that variant's pass over a leading band takes every replica's band
     bool plane_reg = false;      // register first / last passes (every replica's lateral mesh square and supported)
     int flush_kernels = 0;       // kernels per potential-mesh rebuild
     bool unit_pending = false;   // next rebuild places a unit charge instead of the particles
@@ -97,6 +98,7 @@ int zreg_variant(int nz);      // default register z-pass variant for nz, 0 if n
 int zreg_variants(int nz, int* ids, int max_ids);  // every register variant for nz
 void zreg_split(int id, int* n1, int* n2);         // its two stages nz = n1 x n2
 size_t zreg_smem(int nz);
+bool zband_fits(int id, int nz, int zb_lo, int zb_n);  // the split's pass over a leading band takes these planes
 bool plane_reg_supported(int nx, int ny);
 size_t plane_reg_smem(int n);
 
