@@ -526,18 +526,13 @@ static int build(phmc_engine* h, int R, const phmc_system* sys, const phmc_param
             zoff.push_back((int)zj.size());
             zoffr.push_back((int)zjr.size());
             if (E.use_r2c) {
-                // column tiles of near-equal width <= ZPASS_TX over the nx/2+1 half-spectrum columns
-                const int nxh = D.mesh[0] / 2 + 1;
+                // ZREG_TX (ZPASS_TX) consecutive columns of the flattened ny x nxh plane per job
+                const int nxh = D.mesh[0] / 2 + 1, ncol = nxh * D.mesh[1];
                 if (E.zreg_default) {
-                    // ZREG_TX consecutive columns of the flattened ny x nxh plane per job
-                    const int ncol = nxh * D.mesh[1];
                     for (int c0 = 0; c0 < ncol; c0 += ZREG_TX) zjr.push_back(make_int4(r, c0, std::min(ZREG_TX, ncol - c0), 0));
                     E.zpass_smem_reg = std::max(E.zpass_smem_reg, zreg_smem(D.mesh[2]));
                 }
-                const int nt = (nxh + ZPASS_TX - 1) / ZPASS_TX;
-                const int w = (nxh + nt - 1) / nt;
-                for (int y = 0; y < D.mesh[1]; ++y)
-                    for (int x0 = 0; x0 < nxh; x0 += w) zj.push_back(make_int4(r, y, x0, std::min(w, nxh - x0)));
+                for (int c0 = 0; c0 < ncol; c0 += ZPASS_TX) zj.push_back(make_int4(r, c0, std::min(ZPASS_TX, ncol - c0), 0));
                 // band spread: the plane's fixed-point sums; first pass: two complex buffers
                 E.band_spread_smem = std::max(E.band_spread_smem, (size_t)D.mesh[0] * D.mesh[1] * sizeof(unsigned long long));
                 const size_t plane_smem = E.plane_reg ? plane_reg_smem(D.mesh[0]) : (size_t)2 * nxh * D.mesh[1] * sizeof(float2);

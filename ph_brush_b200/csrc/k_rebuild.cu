@@ -14,7 +14,7 @@
 //  k_rb_fwd  (replica, z): Q plane -> float, real-to-complex FFT along x (length
 //            nx/2 complex FFT of packed pairs + split) and complex FFT along y;
 //            writes (nx/2+1) x ny complex values.
-//  k_rb_zpass / k_rb_zreg (column tiles): FFT along z, E += w theta |F|^2,
+//  k_rb_zpass / k_rb_zreg / k_rb_zband (column tiles): FFT along z, E += w theta |F|^2,
 //            F *= theta, inverse FFT along z.
 //  k_rb_inv  (replica, z): inverse FFT along y, complex-to-real along x; writes
 //            the real potential plane.
@@ -219,54 +219,99 @@ __global__ void __launch_bounds__(NT) k_rb_fwd(DevPtrs d, const int2* __restrict
     for (int i = tid; i < nxh * ny; i += NT) c[i] = res[i];
 }
 
-// z pencils of the half spectrum; job = (replica, y, x0, width <= ZPASS_TX).
+// The z pass of any nz = 2^a 3^b 5^c: TX consecutive columns of the flattened half-spectrum plane,
+// job = (replica, first column, columns, 0), Stockham stages of fft_lines' radices, operations and
+// roundings.  A thread stays on one column; the first stage takes its inputs from global memory (without its
+// twiddles, which are one), the last forward stage leaves its outputs times theta, the last
+// inverse stage stores the band's planes: for s stages 2 s - 1 round trips through shared memory
+// instead of 2 s + 3.  Bound by instruction issue and those round trips: 24 uneven replicas (18k
+// columns of 192 to 288 planes) 69 -> 29 us, one without walls (1.9k columns, fewer blocks than SMs) 43 -> 32 us.
+template <int R, bool FIRST, int NT, int TX, class Load, class Store>
+__device__ __forceinline__ void zstage(int n, int Ns, const float2* __restrict__ tw, float sign, Load ld, Store st) {
+    const int nb = n / R, ts = n / (Ns * R);
+    const FastDiv dns(Ns);
+    for (int j = threadIdx.x / TX; j < nb; j += NT / TX) {
+        int k = 0, jq = j;
+        float2 v[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) v[r] = ld(j + r * nb);
+        if constexpr (!FIRST) {
+            jq = dns.div(j, k);
+#pragma unroll
+            for (int r = 1; r < R; ++r) {
+                float2 w = __ldg(&tw[r * k * ts]);
+                if (sign > 0.0f) w.y = -w.y;
+                v[r] = cmul(v[r], w);
+            }
+        }
+        dft_radix(v, R, sign);
+        const int idx = jq * Ns * R + k;
+#pragma unroll
+        for (int r = 0; r < R; ++r) st(idx + r * Ns, v[r]);
+    }
+    __syncthreads();
+}
+
 template <int NT, int TX>
 __global__ void __launch_bounds__(NT) k_rb_zpass(DevPtrs d, const int4* __restrict__ jobs, double* __restrict__ epart,
                                                  const int* __restrict__ dirty, int full) {
+    static_assert(NT % TX == 0, "a thread stays on one column");
     extern __shared__ float2 sm[];
     __shared__ double red[40];
     const int4 job = jobs[blockIdx.x];
-    const int r = job.x, y = job.y, x0 = job.z, tw_n = job.w;
+    const int r = job.x, c0 = job.y, ncol = job.z;
     if (dirty && !dirty[r]) { if (threadIdx.x == 0) epart[blockIdx.x] = 0.0; return; }
     const RepDesc& D = d.desc[r];
-    const int nx = D.mesh[0], ny = D.mesh[1], nz = D.mesh[2];
-    const int M = nx / 2, nxh = M + 1;
-    float2* a = sm;
-    float2* b = sm + TX * nz;
-    float2* c = d.cmesh + D.meshh_off;
-    const int zlo = full ? 0 : D.zb_lo, zbn = full ? nz : D.zb_n;
-    auto in_band = [&](int z) { int t = z - zlo; t += (t < 0) ? nz : 0; return t < zbn; };
-    for (int e = threadIdx.x; e < nz * TX; e += NT) {
-        const int z = e / TX, tx = e - z * TX;
-        a[e] = (tx < tw_n && in_band(z)) ? c[((size_t)z * ny + y) * nxh + x0 + tx] : make_float2(0.f, 0.f);
-    }
-    __syncthreads();
-    float2* res = fft_lines<NT>(a, b, nz, TX, 1, TX, d.twiddle + D.tw_off[2], -1.0f, true);
-    const float2* thx = d.thtab + D.th_off[0];
-    const float2 fy = d.thtab[D.th_off[1] + y];
+    const int nxh = D.mesh[0] / 2 + 1, nz = D.mesh[2], plane = D.mesh[1] * nxh;
+    const int col = threadIdx.x % TX;
+    const bool valid = col < ncol;
+    float2* a = sm + col;
+    float2* b = a + TX * nz;
+    float2* c = d.cmesh + D.meshh_off + c0 + col;
+    const float2* tw = d.twiddle + D.tw_off[2];
     const float2* thz = d.thtab + D.th_off[2];
+    // planes outside the wall band hold no charge (zero input) and are not read back
+    const int zlo = full ? 0 : D.zb_lo, zbn = full ? nz : D.zb_n;
+    auto in_band = [&](int z) { int t = z - zlo; t += (t < 0) ? nz : 0; return valid && t < zbn; };
+    const int idx = c0 + col, y = idx / nxh, kx = idx - y * nxh;
+    const float2 fx = valid ? d.thtab[D.th_off[0] + kx] : make_float2(0.0f, 1.0f);
+    const float2 fy = valid ? d.thtab[D.th_off[1] + y] : make_float2(0.0f, 1.0f);
+    const float cxy = D.th_c * fx.x * fy.x, kxy2 = fx.y + fy.y;
+    const float wgt = (kx == 0 || kx == nxh - 1) ? 1.0f : 2.0f;  // half spectrum, Hermitian partners counted
     double e_loc = 0.0;
-    for (int e = threadIdx.x; e < nz * TX; e += NT) {
-        const int kz = e / TX, tx = e - kz * TX;
-        const int kx = x0 + tx;
-        const float2 F = res[e];
-        float th = 0.0f;
-        if (tx < tw_n && !(kx == 0 && y == 0 && kz == 0)) {
-            // theta = th_c tx ty tz / |k|^2 from the per-axis factor tables
-            const float2 fx = __ldg(&thx[kx]), fz = __ldg(&thz[kz]);
-            th = __fdividef(D.th_c * fx.x * fy.x * fz.x, fx.y + fy.y + fz.y);
-            const float wgt = (kx == 0 || kx == M) ? 1.0f : 2.0f;  // half spectrum, Hermitian partners counted
-            e_loc += (double)(wgt * th) * ((double)F.x * F.x + (double)F.y * F.y);
+    auto global = [&](int z) { return in_band(z) ? c[(size_t)z * plane] : make_float2(0.f, 0.f); };
+    auto shared = [&](int z) { return a[z * TX]; };
+    auto keep = [&](int z, float2 v) { b[z * TX] = v; };
+    auto scale = [&](int kz, float2 F) {  // theta = th_c tx ty tz / |k|^2 from the per-axis factor tables
+        const float2 fz = __ldg(&thz[kz]);
+        float th = __fdividef(cxy * fz.x, kxy2 + fz.y);
+        if (kz == 0 && idx == 0) th = 0.0f;
+        e_loc += (double)(wgt * th) * ((double)F.x * F.x + (double)F.y * F.y);
+        b[kz * TX] = make_float2(__fmul_rn(F.x, th), __fmul_rn(F.y, th));
+    };
+    auto store = [&](int z, float2 v) { if (in_band(z)) c[(size_t)z * plane] = v; };
+    auto stages = [&](float sign, auto first, auto last) {
+        auto one = [&](auto rc, int Ns, int m) {
+            constexpr int R = decltype(rc)::value;
+            if (Ns == 1) {
+                if (m == R) zstage<R, true, NT, TX>(nz, Ns, tw, sign, first, last);
+                else zstage<R, true, NT, TX>(nz, Ns, tw, sign, first, keep);
+            } else if (m == R) zstage<R, false, NT, TX>(nz, Ns, tw, sign, shared, last);
+            else zstage<R, false, NT, TX>(nz, Ns, tw, sign, shared, keep);
+            float2* t = a; a = b; b = t;
+        };
+        for (int Ns = 1, m = nz; m > 1;) {
+            const int R = m % 4 == 0 ? 4 : (m % 2 == 0 ? 2 : (m % 3 == 0 ? 3 : 5));
+            if (R == 4) one(std::integral_constant<int, 4>{}, Ns, m);
+            else if (R == 2) one(std::integral_constant<int, 2>{}, Ns, m);
+            else if (R == 3) one(std::integral_constant<int, 3>{}, Ns, m);
+            else one(std::integral_constant<int, 5>{}, Ns, m);
+            Ns *= R;
+            m /= R;
         }
-        res[e] = make_float2(F.x * th, F.y * th);
-    }
-    __syncthreads();
-    float2* oth = (res == a) ? b : a;
-    res = fft_lines<NT>(res, oth, nz, TX, 1, TX, d.twiddle + D.tw_off[2], 1.0f, true);
-    for (int e = threadIdx.x; e < nz * TX; e += NT) {
-        const int z = e / TX, tx = e - z * TX;
-        if (tx < tw_n && in_band(z)) c[((size_t)z * ny + y) * nxh + x0 + tx] = res[e];
-    }
+    };
+    stages(-1.0f, global, scale);
+    stages(1.0f, shared, store);
     const double s = block_sum<NT>(e_loc, red);
     if (threadIdx.x == 0) epart[blockIdx.x] = 0.5 * s;
 }

@@ -35,3 +35,22 @@ def test_band_pass(nz, order, lift):
             dE[v] = [d["coul_recip"] for d in e.delta_energy_components(moves)]
     for v in SPLITS[nz]:
         assert all(close(a, b, 1e-5, 1e-4) for a, b in zip(dE[v], dE[0]))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nz", [5, 6, 8, 15, 20, 150, 324, 432])
+@pytest.mark.parametrize("nx", [16, 36, 50])
+def test_any_depth(nz, nx):
+    """The Stockham pass: one to six stages of radices 2 to 5, column counts that do not fill a
+    block's sixteen, with walls and without (every plane holds charge)."""
+    for walls in (1, 0):
+        s, p = configs.small_system(seed=nz + nx, mesh=(nx, 18, nz))
+        p.walls = walls
+        ref = O.energy(s, p)
+        with Engine(s, p) as e:
+            if e.tuning()["zpass"]:
+                e.set_tile_shapes(zpass=0)
+            assert_components(e.energy()[0], ref)
+            st = e.run(400)[0]
+            fresh = e.energy()[0]["total"]
+            assert close(st["energy"], fresh, 1e-6, 1e-3)
