@@ -561,6 +561,16 @@ static int build(phmc_engine* h, int R, const phmc_system* sys, const phmc_param
             CU(cudaMemcpy(E.d_zj_reg, zjr.data(), sizeof(int4) * zjr.size(), cudaMemcpyHostToDevice));
             CU(cudaMemcpy(E.d_zoff_reg, zoffr.data(), sizeof(int) * zoffr.size(), cudaMemcpyHostToDevice));
         }
+        if (E.use_r2c) {
+            if (E.nsm == 0) CU(cudaDeviceGetAttribute(&E.nsm, cudaDevAttrMultiProcessorCount, device));
+            E.spread_zp = spread_planes(E.n_band_jobs, (int)(E.band_spread_smem / sizeof(unsigned long long)), E.nsm);
+            std::vector<int2> sj;
+            for (int r = 0; r < R; ++r)
+                for (int i = 0; i < E.desc[r].zb_n; i += E.spread_zp) sj.push_back(make_int2(r, i));
+            E.n_spread_jobs = (int)sj.size();
+            DALLOC(E.d_spread_jobs, sj.size());
+            CU(cudaMemcpy(E.d_spread_jobs, sj.data(), sizeof(int2) * sj.size(), cudaMemcpyHostToDevice));
+        }
         select_zpass(E, E.zreg_default);
         if (E.use_r2c) CU(rebuild_set_smem_limits(E));
         else CU(mesh_set_smem_limits(E));

@@ -38,6 +38,8 @@ struct Engine {
     int2* d_plane_jobs = nullptr;
     int n_band_jobs = 0;
     int2* d_band_jobs = nullptr;  // (replica, z) of the planes in each replica's wall band
+    int spread_zp = 1, n_spread_jobs = 0;
+    int2* d_spread_jobs = nullptr;  // (replica, first band plane) of the spread's blocks
     int4* d_zjobs = nullptr;     // the active z pass's jobs and per-replica job offsets
     int* d_zjob_off = nullptr;
     int4* d_zj_stk = nullptr; int* d_zoff_stk = nullptr; int n_zj_stk = 0;  // shared-memory (Stockham) z pass
@@ -94,6 +96,7 @@ cudaError_t mesh_set_smem_limits(Engine& E);
 void launch_rebuild_r2c(Engine& E, const int* dirty, int unit_charge, cudaStream_t st);
 cudaError_t rebuild_set_smem_limits(Engine& E);
 void launch_band_spread(Engine& E, cudaStream_t st);
+int spread_planes(int n_planes, int np_max, int nsm);  // its planes per block
 int zreg_variant(int nz);      // default register z-pass variant for nz, 0 if none
 int zreg_variants(int nz, int* ids, int max_ids);  // every register variant for nz
 void zreg_split(int id, int* n1, int* n2);         // its two stages nz = n1 x n2

@@ -31,15 +31,16 @@
 #include "fft_reg.cuh"
 #include "fft_packed.cuh"
 
-// One block per (replica, band plane): the charges whose order-P stencils reach the plane, from the
-// cell list, added into a fixed-point plane in shared memory.  A value (2^-40 units, 41 bits) is
+// One block per (replica, ZP consecutive band planes): the charges whose order-P stencils reach
+// them, from the cell list, added into fixed-point planes in shared memory.  A value (2^-40 units, 41 bits) is
 // added as two 32-bit halves, its low 20 bits and the rest, since 64-bit adds in shared memory are
-// compare-and-swap loops; the halves hold the sums of 4095 charges of 9000 units in all, and a
-// plane that more reach is done over with 64-bit adds.  A warp takes 32 cells at a time, one per
+// compare-and-swap loops; the halves hold the sums of 4095 charges of 9000 units in all, and
+// planes that more reach are done over with 64-bit adds.  A warp takes 32 cells at a time, one per
 // lane for the counts, then one lane per member; those that reach the plane (~40 %) queue up and
-// are added 32 at a time: instruction issue bounds it.  Measured on 64 replicas of 8.7k particles: 300 us
-// with 64-bit adds, 262 us as global integer adds, 195 us; one replica of 11.7k: 40 -> 24 us.
-template <int P, int NT>
+// are added 32 at a time: issue and the adds' bank conflicts bound it (half of either's peak).  Measured on 64 replicas of 8.7k particles: 300 us
+// with 64-bit adds, 262 us as global integer adds, 197 us in 32-bit halves, 182 us two planes at a
+// time; of 5k: 143 us, 119 us four planes at a time; one replica of 11.7k: 40 -> 24 us.
+template <int P, int ZP, int NT>
 __global__ void __launch_bounds__(NT) k_band_spread(DevPtrs d, const int2* __restrict__ jobs) {
     extern __shared__ __align__(16) unsigned char sm_raw[];
     constexpr int NW = NT / 32;
@@ -47,17 +48,20 @@ __global__ void __launch_bounds__(NT) k_band_spread(DevPtrs d, const int2* __res
     __shared__ int s_n;
     __shared__ float s_qsum;
     const int2 job = jobs[blockIdx.x];
-    const int r = job.x, z = job.y;
+    const int r = job.x;
     const RepDesc& D = d.desc[r];
     const int nx = D.mesh[0], ny = D.mesh[1], nz = D.mesh[2], np = nx * ny;
+    const int planes = ZP > 1 ? min(ZP, D.zb_n - job.y) : 1;  // band planes job.y .. job.y + planes - 1
+    const int z = D.zb_lo + job.y - (D.zb_lo + job.y >= nz ? nz : 0);
+    const int all = planes * np;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     float4* queue = s_queue[warp];
     unsigned* s_lo = reinterpret_cast<unsigned*>(sm_raw);
-    int* s_hi = reinterpret_cast<int*>(sm_raw) + np;
+    int* s_hi = reinterpret_cast<int*>(sm_raw) + all;
     unsigned long long* s_64 = reinterpret_cast<unsigned long long*>(sm_raw);
-    // floor(g_z) of a contributing charge lies in [z - P/2, z - P/2 + P - 1] (mod nz)
+    // floor(g_z) of a contributing charge lies in [z - P/2, z + planes - 1 - P/2 + P - 1] (mod nz)
     const float hz = D.L[2] / (float)nz;
-    const float zlo = (float)(z - P / 2) * hz, zhi = (float)(z - P / 2 + P) * hz;
+    const float zlo = (float)(z - P / 2) * hz, zhi = (float)(z + planes - 1 - P / 2 + P) * hz;
     const int ncz = D.ncell[2], ncxy = D.ncell[0] * D.ncell[1];
     // the cell layers of [zlo, zhi), widened by a rounding margin (the exact test is per charge)
     int c_lo = (int)floorf((zlo - 1e-3f * hz) * D.cell_scale[2]), c_hi = (int)floorf((zhi + 1e-3f * hz) * D.cell_scale[2]);
@@ -67,7 +71,7 @@ __global__ void __launch_bounds__(NT) k_band_spread(DevPtrs d, const int2* __res
     c_lo += (c_lo < 0) ? ncz : 0;
     const int ncell = nlay * ncxy;
     for (int wide = 0; wide < 2; ++wide) {
-        for (int i = tid; i < np; i += NT) s_64[i] = 0ull;
+        for (int i = tid; i < all; i += NT) s_64[i] = 0ull;
         if (tid == 0) { s_n = 0; s_qsum = 0.0f; }
         __syncthreads();
         int n_in = 0, nh = 0;
@@ -79,9 +83,6 @@ __global__ void __launch_bounds__(NT) k_band_spread(DevPtrs d, const int2* __res
             int ci = z - base[2];
             ci %= nz;
             ci += (ci < 0) ? nz : 0;
-            float wz = 0.0f;  // select: w[2][ci] without a dynamic index
-#pragma unroll
-            for (int j = 0; j < P; ++j) wz = (j == ci) ? w[2][j] : wz;
             ++n_in;
             q_in += fabsf(pq.w);
             int xa[P];
@@ -91,18 +92,27 @@ __global__ void __launch_bounds__(NT) k_band_spread(DevPtrs d, const int2* __res
                 xa[aa] += (xa[aa] < 0) ? nx : 0;
                 xa[aa] -= (xa[aa] >= nx) ? nx : 0;
             }
+            for (int q = 0; q < planes; ++q) {  // (one plane: no loop)
+                int cq = ci + q;
+                cq -= (cq >= nz) ? nz : 0;
+                if (ZP > 1 && cq >= P) continue;
+                float wz = 0.0f;  // select: w[2][cq] without a dynamic index
 #pragma unroll
-            for (int bb = 0; bb < P; ++bb) {
-                int yb = base[1] + bb;
-                yb += (yb < 0) ? ny : 0;
-                yb -= (yb >= ny) ? ny : 0;
+                for (int j = 0; j < P; ++j) wz = (j == cq) ? w[2][j] : wz;
 #pragma unroll
-                for (int aa = 0; aa < P; ++aa) {
-                    const long long v = qmesh_value(pq.w, w[0][aa], w[1][bb], wz);
-                    if (wide) atomicAdd(&s_64[yb * nx + xa[aa]], (unsigned long long)v);
-                    else {
-                        atomicAdd(&s_lo[yb * nx + xa[aa]], (unsigned)(v & 0xfffff));
-                        atomicAdd(&s_hi[yb * nx + xa[aa]], (int)(v >> 20));
+                for (int bb = 0; bb < P; ++bb) {
+                    int yb = base[1] + bb;
+                    yb += (yb < 0) ? ny : 0;
+                    yb -= (yb >= ny) ? ny : 0;
+                    yb = q * np + yb * nx;
+#pragma unroll
+                    for (int aa = 0; aa < P; ++aa) {
+                        const long long v = qmesh_value(pq.w, w[0][aa], w[1][bb], wz);
+                        if (wide) atomicAdd(&s_64[yb + xa[aa]], (unsigned long long)v);
+                        else {
+                            atomicAdd(&s_lo[yb + xa[aa]], (unsigned)(v & 0xfffff));
+                            atomicAdd(&s_hi[yb + xa[aa]], (int)(v >> 20));
+                        }
                     }
                 }
             }
@@ -138,7 +148,7 @@ __global__ void __launch_bounds__(NT) k_band_spread(DevPtrs d, const int2* __res
                         int ci = z - ((int)floorf(__fmul_rn(__fdiv_rn(pq.z, D.L[2]), (float)nz)) + P / 2 - P + 1);
                         ci %= nz;
                         ci += (ci < 0) ? nz : 0;
-                        hit = ci < P;
+                        hit = ci < P || ci + planes > nz;
                     }
                 }
                 const unsigned hm = __ballot_sync(0xffffffffu, hit);
@@ -158,12 +168,10 @@ __global__ void __launch_bounds__(NT) k_band_spread(DevPtrs d, const int2* __res
         if (lane < nh) add(queue[lane]);
         if (n_in) { atomicAdd(&s_n, n_in); atomicAdd(&s_qsum, q_in); }
         __syncthreads();
-        int zrel = z - D.zb_lo;
-        zrel += (zrel < 0) ? nz : 0;
-        unsigned long long* q = d.qband + D.qb_off + (size_t)zrel * np;
+        unsigned long long* q = d.qband + D.qb_off + (size_t)job.y * np;
         const bool fits = s_n <= 4095 && s_qsum <= 9000.0f;
         if (wide || fits) {
-            for (int i = tid; i < np; i += NT)
+            for (int i = tid; i < all; i += NT)
                 q[i] = wide ? s_64[i] : (unsigned long long)(((long long)s_hi[i] << 20) + (long long)s_lo[i]);
             return;
         }
@@ -904,13 +912,36 @@ void launch_rebuild_r2c(Engine& E, const int* dirty, int unit_charge, cudaStream
     else k_rb_inv<256><<<npj, 256, E.rb_inv_smem, st>>>(E.d, pj, dirty);
 }
 
+// Planes per block of the spread: a charge is found and its weights are made once per block that it
+// reaches, (ZP + P - 1) / ZP times per plane, so as many as leave three blocks to an SM; one where
+// the band's planes would not fill the device with four blocks to an SM.
+int spread_planes(int n_planes, int np_max, int nsm) {
+    int zp = 1;
+    while (zp < 4 && (size_t)(zp + 1) * np_max * 8 <= 72 * 1024 && n_planes >= 4 * nsm * (zp + 1)) ++zp;
+    return zp;
+}
+
+template <class F>
+static void spread_dispatch(const Engine& E, F&& f) {
+    auto planes = [&](auto p) {
+        switch (E.spread_zp) {
+            case 1: f(p, std::integral_constant<int, 1>{}); break;
+            case 2: f(p, std::integral_constant<int, 2>{}); break;
+            case 3: f(p, std::integral_constant<int, 3>{}); break;
+            default: f(p, std::integral_constant<int, 4>{}); break;
+        }
+    };
+    if (E.order == 4) planes(std::integral_constant<int, 4>{});
+    else if (E.order == 5) planes(std::integral_constant<int, 5>{});
+    else planes(std::integral_constant<int, 6>{});
+}
+
 // Charge mesh of every replica's wall band from scratch (full recompute).
 void launch_band_spread(Engine& E, cudaStream_t st) {
-    switch (E.order) {
-        case 4: k_band_spread<4, 256><<<E.n_band_jobs, 256, E.band_spread_smem, st>>>(E.d, E.d_band_jobs); break;
-        case 5: k_band_spread<5, 256><<<E.n_band_jobs, 256, E.band_spread_smem, st>>>(E.d, E.d_band_jobs); break;
-        default: k_band_spread<6, 256><<<E.n_band_jobs, 256, E.band_spread_smem, st>>>(E.d, E.d_band_jobs); break;
-    }
+    spread_dispatch(E, [&](auto p, auto zp) {
+        k_band_spread<decltype(p)::value, decltype(zp)::value, 256>
+            <<<E.n_spread_jobs, 256, E.spread_zp * E.band_spread_smem, st>>>(E.d, E.d_spread_jobs);
+    });
 }
 
 template <typename K>
@@ -928,11 +959,9 @@ static cudaError_t raise_cap(K kernel, int device, size_t need) {
 
 cudaError_t rebuild_set_smem_limits(Engine& E) {
     cudaError_t e = cudaSuccess;
-    switch (E.order) {
-        case 4: e = raise_cap(k_band_spread<4, 256>, E.device, E.band_spread_smem); break;
-        case 5: e = raise_cap(k_band_spread<5, 256>, E.device, E.band_spread_smem); break;
-        default: e = raise_cap(k_band_spread<6, 256>, E.device, E.band_spread_smem); break;
-    }
+    spread_dispatch(E, [&](auto p, auto zp) {
+        e = raise_cap(k_band_spread<decltype(p)::value, decltype(zp)::value, 256>, E.device, E.spread_zp * E.band_spread_smem);
+    });
     if (e != cudaSuccess) return e;
     e = E.plane_reg ? raise_cap(k_rb_fwd_reg<PLANE_NT>, E.device, E.rb_fwd_smem) : raise_cap(k_rb_fwd<256>, E.device, E.rb_fwd_smem);
     if (e != cudaSuccess) return e;
