@@ -39,7 +39,7 @@
 // lane for the counts, then one lane per member; those that reach the plane (~40 %) queue up and
 // are added 32 at a time: issue and the adds' bank conflicts bound it (half of either's peak).  Measured on 64 replicas of 8.7k particles: 300 us
 // with 64-bit adds, 262 us as global integer adds, 197 us in 32-bit halves, 182 us two planes at a
-// time; of 5k: 143 us, 119 us four planes at a time; one replica of 11.7k: 40 -> 24 us.
+// time; of 5k: 143 us, 111 us three planes at a time; one replica of 11.7k: 40 -> 24 us.
 template <int P, int ZP, int NT>
 __global__ void __launch_bounds__(NT) k_band_spread(DevPtrs d, const int2* __restrict__ jobs) {
     extern __shared__ __align__(16) unsigned char sm_raw[];
@@ -913,11 +913,12 @@ void launch_rebuild_r2c(Engine& E, const int* dirty, int unit_charge, cudaStream
 }
 
 // Planes per block of the spread: a charge is found and its weights are made once per block that it
-// reaches, (ZP + P - 1) / ZP times per plane, so as many as leave three blocks to an SM; one where
-// the band's planes would not fill the device with four blocks to an SM.
+// reaches, (ZP + P - 1) / ZP times per plane, so as many as leave three blocks to an SM (the block's
+// queues take 8 KB more; four planes of 48 x 48 leave two and take 119 us where three take 111); one
+// where the band's planes would not fill the device with four blocks to an SM.
 int spread_planes(int n_planes, int np_max, int nsm) {
     int zp = 1;
-    while (zp < 4 && (size_t)(zp + 1) * np_max * 8 <= 72 * 1024 && n_planes >= 4 * nsm * (zp + 1)) ++zp;
+    while (zp < 4 && (size_t)(zp + 1) * np_max * 8 <= 64 * 1024 && n_planes >= 4 * nsm * (zp + 1)) ++zp;
     return zp;
 }
 
