@@ -18,7 +18,9 @@
 // A batch ends early (and the next one starts there) where an accepted trial could have
 // changed a later one: an inserted or removed particle changes the index lists that
 // proposals draw from; a changed particle within the largest cutoff of a later trial's
-// probe, or bonded to its particle, changes that trial's pair terms.  What remains is
+// probe, or bonded to its particle, changes that trial's pair terms; and a moved particle
+// that a later trial displaces again, also one that the walls refused from the old place,
+// changes that trial.  What remains is
 // exactly the sequence of one-at-a-time trials, and because every sum is formed per probe
 // and per stencil pair in a fixed order, its energies are bit for bit independent of the
 // batch's size and of the block's number of warps.
@@ -416,9 +418,10 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_mc_run(DevPtrs d, int pend_max
                     t.direct_lj = dl; t.direct_c = dc;
                     t.dQ = dQ; t.dQ2 = dQ2; t.dMz = dMz; t.dS2 = dS2;
                 }
-            } else {  // would trial i, accepted, change trial j's pair or bond terms?
+            } else {  // would trial i, accepted, change trial j's pair or bond terms, or its wall verdict?
+                // (a refused trial j has no probes: only the particles are compared)
                 const int i = (it - Q_CF) / RUN_BATCH, j = (it - Q_CF) % RUN_BATCH;
-                if (i < j && j < nb && B.T[i].skip == 0 && B.T[j].skip == 0) {
+                if (i < j && j < nb && B.T[i].skip == 0 && (B.T[j].skip == 0 || B.T[j].skip == 2)) {
                     const RunTrial &a = B.T[i], &b = B.T[j];
                     bool hit = false;
                     for (int p = a.p0; p < a.p0 + a.np && !hit; ++p)
@@ -430,7 +433,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_mc_run(DevPtrs d, int pend_max
                         }
                     for (int k = 0; k < a.nch; ++k)
                         for (int l = 0; l < b.nch; ++l)
-                            hit = hit || a.idx[k] == b.idx[l] || in_bonds(b.bonds[l], a.idx[k]);
+                            hit = hit || a.idx[k] == b.idx[l] || (b.skip == 0 && in_bonds(b.bonds[l], a.idx[k]));
                     if (hit) atomicOr(&s_conf[i], 1u << j);
                 }
             }
