@@ -31,11 +31,16 @@
 #include "fft_reg.cuh"
 #include "fft_packed.cuh"
 
+// sum of |q| up to which a block of the spread adds in 32-bit halves
+constexpr float spread_qmax(int order) { return order == 4 ? 6900.0f : 9000.0f; }
+
 // One block per (replica, ZP consecutive band planes): the charges whose order-P stencils reach
 // them, from the cell list, added into fixed-point planes in shared memory.  A value (2^-40 units, 41 bits) is
 // added as two 32-bit halves, its low 20 bits and the rest, since 64-bit adds in shared memory are
-// compare-and-swap loops; the halves hold the sums of 4095 charges of 9000 units in all, and
-// planes that more reach are done over with 64-bit adds.  A warp takes 32 cells at a time, one per
+// compare-and-swap loops.  The low halves hold the sums of 4095 charges; the upper ones hold |q| w^3 2^20
+// below 2^31 at a point, w the largest 1-D weight (2/3, 115/192, 11/20 at order 4, 5, 6): 6912, 9531,
+// 12309 units in all.  Planes that more reach (spread_qmax: a little less, for the roundings down
+// and the FP32 sum of |q|) are done over with 64-bit adds.  A warp takes 32 cells at a time, one per
 // lane for the counts, then one lane per member; those that reach the plane (~40 %) queue up and
 // are added 32 at a time: issue and the adds' bank conflicts bound it (half of either's peak).  Measured on 64 replicas of 8.7k particles: 300 us
 // with 64-bit adds, 262 us as global integer adds, 197 us in 32-bit halves, 182 us two planes at a
@@ -169,7 +174,7 @@ __global__ void __launch_bounds__(NT) k_band_spread(DevPtrs d, const int2* __res
         if (n_in) { atomicAdd(&s_n, n_in); atomicAdd(&s_qsum, q_in); }
         __syncthreads();
         unsigned long long* q = d.qband + D.qb_off + (size_t)job.y * np;
-        const bool fits = s_n <= 4095 && s_qsum <= 9000.0f;
+        const bool fits = s_n <= 4095 && s_qsum <= spread_qmax(P);
         if (wide || fits) {
             for (int i = tid; i < all; i += NT)
                 q[i] = wide ? s_64[i] : (unsigned long long)(((long long)s_hi[i] << 20) + (long long)s_lo[i]);
