@@ -732,6 +732,7 @@ extern "C" int phmc_energy(phmc_engine* h, phmc_energy_components* out) {
 }
 
 static int check_trials(phmc_engine* h, int rep, const phmc_trial* t, int n) {
+    if (n < 0) return fail(PHMC_ERR_ARG, "negative number of trials");
     if (rep < 0 || rep >= h->E.R) return fail(PHMC_ERR_ARG, "replica index out of range");
     for (int k = 0; k < n; ++k) {
         if (t[k].n_changes < 1 || t[k].n_changes > 2) return fail(PHMC_ERR_ARG, "trial must have 1 or 2 changes");
@@ -757,13 +758,11 @@ static int ensure_trial_buffers(phmc_engine* h, int n) {
     return PHMC_OK;
 }
 
-// Judge n external trials: their dE (res[0 .. n)) and, with comps, 7 components each after them.
+// Judge n external trials (checked): their dE (res[0 .. n)) and, with comps, 7 components each after them.
 static int judge_trials(phmc_engine* h, int rep, const phmc_trial* trials, int n, bool comps, double* res) {
-    int s = check_trials(h, rep, trials, n);
-    if (s) return s;
     Engine& E = h->E;
     CU(cudaSetDevice(E.device));
-    s = ensure_trial_buffers(h, n);
+    int s = ensure_trial_buffers(h, n);
     if (s) return s;
     const bool pin = n <= PIN_TRIALS;
     const size_t bytes = sizeof(double) * (comps ? 8 : 1) * (size_t)n;
@@ -791,7 +790,8 @@ static int flush_dirty(phmc_engine* h) {
 extern "C" int phmc_delta_energy(phmc_engine* h, int rep, const phmc_trial* trials, int n, double* dE) {
     if (!h || (n > 0 && (!trials || !dE))) return fail(PHMC_ERR_ARG, "null argument");
     if (n == 0) return PHMC_OK;
-    return judge_trials(h, rep, trials, n, false, dE);
+    const int s = check_trials(h, rep, trials, n);
+    return s ? s : judge_trials(h, rep, trials, n, false, dE);
 }
 
 extern "C" int phmc_commit(phmc_engine* h, int rep, const phmc_trial* trial) {
@@ -2091,9 +2091,11 @@ extern "C" int phmc_autotune(phmc_engine* h, int64_t trials, phmc_tuning* result
 extern "C" int phmc_delta_energy_components(phmc_engine* h, int rep, const phmc_trial* trials, int n,
                                             phmc_energy_components* out) {
     if (!h || (n > 0 && (!trials || !out))) return fail(PHMC_ERR_ARG, "null argument");
-    if (n <= 0) return PHMC_OK;
+    if (n == 0) return PHMC_OK;
+    int s = check_trials(h, rep, trials, n);
+    if (s) return s;
     std::vector<double> res((size_t)8 * n);
-    const int s = judge_trials(h, rep, trials, n, true, res.data());
+    s = judge_trials(h, rep, trials, n, true, res.data());
     for (int k = 0; k < n && (s == PHMC_OK || s == PHMC_ERR_CAPACITY); ++k) {
         const double* c = res.data() + n + 7 * (size_t)k;
         out[k].lj = c[0]; out[k].fene = c[1]; out[k].coul_real = c[2]; out[k].coul_recip = c[3];
