@@ -752,6 +752,7 @@ static int check_trials(phmc_engine* h, int rep, const phmc_trial* t, int n) {
 static int ensure_trial_buffers(phmc_engine* h, int n) {
     if (n <= h->trials_cap) return PHMC_OK;
     if (h->d_trials) { cudaFree(h->d_trials); cudaFree(h->d_dE); h->d_trials = nullptr; h->d_dE = nullptr; }
+    h->trials_cap = 0;  // (also where an allocation below fails)
     CU(cudaMalloc((void**)&h->d_trials, sizeof(phmc_trial) * n));
     CU(cudaMalloc((void**)&h->d_dE, sizeof(double) * 8 * (size_t)n));
     h->trials_cap = n;
