@@ -249,6 +249,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_mc_run(DevPtrs d, int pend_max
     lane_place<P>(L, D, lane);
 
     for (;;) {
+        bool halt = false;
         if (rank == 0) {
         // ---------------- proposals ----------------
         if (warp == 0) {
@@ -343,7 +344,10 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_mc_run(DevPtrs d, int pend_max
         __syncthreads();
         mark(0);
         mark(1);
-        if (!B.stop) {
+        // the last batch's moves overflowed a cell while this one was drawn: it is dropped
+        halt = B.stop || S.error;
+        if (tid == 0 && halt) { B.stop = 1; B.ns = 0; }
+        if (!halt) {
         const int nb = B.nb, npend = B.npend, ns = B.ns;
         // ---------------- stencils, direct and bonded terms, conflicts ----------------
         if (tid == 0) s_nq = 0;
@@ -453,10 +457,11 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_mc_run(DevPtrs d, int pend_max
                 const int nv = (int)((sizeof(PadSt<P>) * (n0 + n1) + 15) / 16);
                 for (int k = tid; k < nv; k += NT) sd[k] = ss[k];
                 __syncthreads();
+                halt = B.stop;
             }
-            if (B.stop) break;
+            if (halt) break;
         } else {
-            if (B.stop) break;
+            if (halt) break;
             __syncthreads();
         }
         mark(2);
