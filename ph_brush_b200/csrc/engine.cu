@@ -441,10 +441,10 @@ static int build(phmc_engine* h, int R, const phmc_system* sys, const phmc_param
     DALLOC(E.d_cell_rep, E.total_cells);
     int maxcap = 0;
     for (int r = 0; r < R; ++r) maxcap = std::max(maxcap, E.desc[r].cap);
-    E.energy_blocks = std::max(1, std::min(PHMC_FULL_MAX_BPR, (maxcap + 127) / 128));
     E.max_cap = maxcap;
     for (const RepDesc& D : E.desc) E.max_cells = std::max(E.max_cells, D.ncell[0] * D.ncell[1] * D.ncell[2]);
-    DALLOC(d.partials, (size_t)R * PHMC_FULL_MAX_BPR * 8);  // any energy_block's blocks per replica
+    CU(cudaDeviceGetAttribute(&E.nsm, cudaDevAttrMultiProcessorCount, device));
+    DALLOC(d.partials, full_energy_partials(E));
     DALLOC(E.d_active, 1);
     {
         auto up = [](size_t v) { return (v + 63) / 64 * 64; };
@@ -562,7 +562,6 @@ static int build(phmc_engine* h, int R, const phmc_system* sys, const phmc_param
             CU(cudaMemcpy(E.d_zoff_reg, zoffr.data(), sizeof(int) * zoffr.size(), cudaMemcpyHostToDevice));
         }
         if (E.use_r2c) {
-            if (E.nsm == 0) CU(cudaDeviceGetAttribute(&E.nsm, cudaDevAttrMultiProcessorCount, device));
             E.spread_zp = spread_planes(E.n_band_jobs, (int)(E.band_spread_smem / sizeof(unsigned long long)), E.nsm);
             std::vector<int2> sj;
             for (int r = 0; r < R; ++r)

@@ -64,7 +64,6 @@ struct Engine {
     int* h_active = nullptr;     // pinned mirror
     // full-energy scratch
     double* d_epair = nullptr;   // per (replica, block) partial components
-    int energy_blocks = 0;
     int max_cap = 0;             // largest replica capacity (slots)
     int max_cells = 0;           // largest replica's cell count
     // host copies for trial logs
@@ -108,6 +107,7 @@ size_t plane_reg_smem(int n);
 // k_pair.cu
 void launch_cell_build(Engine& E, cudaStream_t st);
 void launch_full_energy(Engine& E, cudaStream_t st);
+size_t full_energy_partials(const Engine& E);  // its partial sums (doubles), at any energy_block
 
 // k_mlp.cu (surrogate network)
 int sur_device_view(phmc_surrogate* h, SurDev* out);

@@ -331,13 +331,22 @@ __global__ void __launch_bounds__(NT) k_full_reduce(DevPtrs d, int bpr) {
     S.E = S.E_pair_lj + S.E_pair_c + S.E_fene + S.E_rec + S.E_self + S.E_qcorr + S.E_slab;
 }
 
-// E.energy_block (64, 128, 256 threads; 0: 256) is a tuning parameter.  Enough blocks per replica
-// for one cell per warp, while all replicas' blocks stay within about four waves of the chip (the
-// rest of the cells in turn); PHMC_FULL_MAX_BPR bounds the partial sums' size.
+// Blocks per replica at nt threads each: one cell per warp, while all replicas' blocks stay within
+// about four waves of the chip (the rest of the cells in turn), at most PHMC_FULL_MAX_BPR.
+static int full_energy_bpr(const Engine& E, int nt) {
+    const int want = (E.max_cells + nt / 32 - 1) / (nt / 32), room = std::max(8, 4 * E.nsm * 4 * 256 / nt / E.R);
+    return std::max(1, std::min({PHMC_FULL_MAX_BPR, want, room}));
+}
+
+size_t full_energy_partials(const Engine& E) {
+    const int bpr = std::max({full_energy_bpr(E, 64), full_energy_bpr(E, 128), full_energy_bpr(E, 256)});
+    return (size_t)E.R * bpr * 8;
+}
+
+// E.energy_block (64, 128, 256 threads; 0: 256) is a tuning parameter.
 void launch_full_energy(Engine& E, cudaStream_t st) {
     const int nt = E.energy_block ? E.energy_block : 256;
-    const int want = (E.max_cells + nt / 32 - 1) / (nt / 32), room = std::max(8, 4 * 148 * 4 * 256 / nt / E.R);
-    const int bpr = std::max(1, std::min({PHMC_FULL_MAX_BPR, want, room}));
+    const int bpr = full_energy_bpr(E, nt);
     dim3 grid(bpr, E.R);
     if (nt == 64) k_full_energy<64><<<grid, 64, 0, st>>>(E.d, bpr);
     else if (nt == 256) k_full_energy<256><<<grid, 256, 0, st>>>(E.d, bpr);
