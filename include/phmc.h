@@ -213,8 +213,8 @@ int phmc_set_move_mix(phmc_engine* e, int replica, double p_disp, double p_titr,
  * mesh); threads: threads per replica block of the MC kernel (128 or 256).
  * Both may change between runs.  phmc_autotune times `trials` trials per
  * replica for each candidate (pending_max 8..128 x threads 128/256) in two
- * interleaved passes, keeps the fastest and reports every candidate's better time; its runs are ordinary Monte Carlo
- * trials and advance the chains.  Decisions do not depend on the tuning except
+ * interleaved passes, keeps the fastest and reports every candidate's better time; its runs are
+ * ordinary Monte Carlo trials and advance the chains.  Decisions do not depend on the tuning except
  * through FP32 rounding of the reciprocal-space dE. */
 typedef struct phmc_tuning {
     int pending_max;
@@ -255,7 +255,10 @@ int phmc_set_first_stage(phmc_engine* e, int on);
  * interleaved passes, each candidate's faster time kept), then the pair pass's
  * shape (round width x G rows) at the best pending_max x threads, then, with a surrogate attached,
  * its first stage on against bypassed; keeps the fastest of each stage.
- * results[] gets one entry per candidate timed, with that stage's time set. */
+ * results[] gets one entry per candidate, with that stage's time set; candidates that launch the
+ * same code (threads with at most one replica per SM, the pair pass's shape in plain runs and its
+ * g_rows in all, energy_block 0 and 256) share one timing, and the first of them is kept: for
+ * threads the value in force. */
 int phmc_autotune(phmc_engine* e, int64_t trials, phmc_tuning* results, int max_results, int* n_results);
 /* Launch quorum, 0 < quorum <= 1: an MC launch of a batched engine ends once that
  * fraction of the replicas still running at its start have filled their pending

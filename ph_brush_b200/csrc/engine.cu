@@ -1974,28 +1974,38 @@ extern "C" int phmc_autotune(phmc_engine* h, int64_t trials, phmc_tuning* result
         if (s) return s;
     }
     // 2. full recompute's block size (pair / FENE pass and its reduction; the tracked
-    //    pair energies it rewrites are those of the current state)
+    //    pair energies it rewrites are those of the current state); 0 launches 256 threads
     {
         const int blocks[4] = {0, 64, 128, 256};
         int best_b = E.energy_block;
-        double best = 1e300;
+        double best = 1e300, ms_0 = 0.0;
         for (int b : blocks) {
             apply_tiles(h, -1, -1, b);
-            double ms = 0.0;
-            int s = time_launches(E, 5, [&]() { launch_full_energy(E, E.stream); }, &ms);
-            if (s) return s;
+            double ms = ms_0;
+            if (b != 256) {
+                int s = time_launches(E, 5, [&]() { launch_full_energy(E, E.stream); }, &ms);
+                if (s) return s;
+                if (b == 0) ms_0 = ms;
+            }
             emit(0.0, 0.0, ms * 1e3);
             if (ms < best) { best = ms; best_b = b; }
         }
         apply_tiles(h, -1, -1, best_b);
     }
+    // What a run takes notice of.  Candidates that launch the same code share one timing (timed one
+    // by one, noise would choose among them), the first of them in the list is kept: for the block
+    // size the one in force, which external trials go on using.
+    const bool block_size = E.R > E.nsm;  // (otherwise a replica takes blocks of 512 threads)
+    const bool round_width = (E.d.sur.H > 0 && !E.first_stage_off) || E.d.hv_cap > 0;  // (first stage, harvest)
     // 3. pending capacity x block size by trial runs; two passes over the candidates, each
     //    candidate's faster one kept: the chains move on while the tuner runs, and
     //    interleaving keeps that drift from favouring one candidate
-    const int pends[] = {8, 16, 24, 32, 48, 64, 96, 128};
-    const int ths[] = {128, 256};
-    std::vector<double> best_us(16, 1e300);
-    std::vector<char> fits(16, 0);
+    constexpr int NP = 8, NC = 2 * NP;
+    const int pends[NP] = {8, 16, 24, 32, 48, 64, 96, 128};
+    const int ths[2] = {E.threads, E.threads == 128 ? 256 : 128};
+    double best_us[NC];
+    bool fits[NC] = {false};
+    std::fill(best_us, best_us + NC, 1e300);
     auto time_run = [&](double* us) -> int {
         int s = phmc_run_loop(h, std::max<int64_t>(trials / 4, 4), 4);  // warm-up (captures the graph)
         if (s) return s;
@@ -2005,50 +2015,44 @@ extern "C" int phmc_autotune(phmc_engine* h, int64_t trials, phmc_tuning* result
         *us = ms * 1e3 / (double)trials;
         return PHMC_OK;
     };
-    for (int pass = 0; pass < 2; ++pass) {
-        int c = 0;
-        for (int th : ths)
-            for (int pm : pends) {
-                const int k = c++;
-                if (pm > PHMC_MAX_PEND || (pass == 1 && !fits[k])) continue;
-                if (apply_tuning(h, pm, th) != PHMC_OK) continue;  // does not fit: skip
-                fits[k] = 1;
-                double us = 0.0;
-                int s = time_run(&us);
-                if (s) return s;
-                best_us[k] = std::min(best_us[k], us);
-            }
-    }
-    int best_p = E.pend_max, best_t = E.threads, c = 0;
+    for (int pass = 0; pass < 2; ++pass)
+        for (int k = 0; k < NC; ++k) {
+            const int pm = pends[k % NP];
+            if (pm > PHMC_MAX_PEND || (pass == 1 && !fits[k])) continue;
+            if (apply_tuning(h, pm, ths[k / NP]) != PHMC_OK) continue;  // does not fit: skip
+            fits[k] = true;
+            if (!block_size && k >= NP && fits[k - NP]) { best_us[k] = best_us[k - NP]; continue; }
+            double us = 0.0;
+            int s = time_run(&us);
+            if (s) return s;
+            best_us[k] = std::min(best_us[k], us);
+        }
+    int best_p = E.pend_max, best_t = E.threads;
     double best = 1e300;
-    for (int th : ths)
-        for (int pm : pends) {
-            const int k = c++;
-            if (!fits[k]) continue;
-            if (best_us[k] < best) { best = best_us[k]; best_p = pm; best_t = th; }
+    for (int k = 0; k < NC; ++k)
+        if (fits[k] && best_us[k] < best) { best = best_us[k]; best_p = pends[k % NP]; best_t = ths[k / NP]; }
+    for (int k = 0; k < NC; ++k) {
+        if (!fits[k]) continue;
+        if (results && n < max_results) {
+            fill_tuning(E, &results[n]);
+            results[n].pending_max = pends[k % NP]; results[n].threads = ths[k / NP]; results[n].us_per_trial = best_us[k];
         }
-    c = 0;
-    for (int th : ths)
-        for (int pm : pends) {
-            const int k = c++;
-            if (!fits[k]) continue;
-            if (results && n < max_results) {
-                fill_tuning(E, &results[n]);
-                results[n].pending_max = pm; results[n].threads = th; results[n].us_per_trial = best_us[k];
-            }
-            ++n;
-        }
+        ++n;
+    }
     int s = apply_tuning(h, best_p, best_t);
     if (s) return s;
     // 4. the pair pass's shape at that pending capacity and block size (order 5): round width
-    //    (candidates per thread per round) x G rows in flight in the correction sum
+    //    (candidates per thread per round) x G rows, which no run takes notice of
     if (E.order == 5) {
-        const int shapes[7][2] = {{4, 2}, {2, 2}, {8, 2}, {2, 3}, {2, 4}, {2, 21}, {4, 21}};
         constexpr int NSH = 7;
+        const int shapes[NSH][2] = {{4, 2}, {2, 2}, {8, 2}, {2, 3}, {2, 4}, {2, 21}, {4, 21}};
+        const int as[NSH] = {0, 1, 2, 1, 1, 1, 0};  // the first shape of the same width
         double sbest[NSH] = {best, 1e300, 1e300, 1e300, 1e300, 1e300, 1e300};
         for (int pass = 0; pass < 2; ++pass)
             for (int k = 1; k < NSH; ++k) {
                 if (apply_tiles(h, -1, shapes[k][0], -1, shapes[k][1]) != PHMC_OK) continue;
+                const int same = round_width ? as[k] : 0;
+                if (same != k && sbest[same] < 1e300) { sbest[k] = sbest[same]; continue; }
                 double us = 0.0;
                 s = time_run(&us);
                 if (s) return s;
