@@ -240,7 +240,8 @@ def barrier(world):
 
 def tune_engine(eng, args, trials):
     """Autotune, or apply --tuning pending_max,threads[,cand_round,g_rows,zpass,plane_pipe,first_stage]
-    (fixed shapes for profiling commands; -1 keeps a field)."""
+    (fixed shapes for profiling commands; -1 keeps a field).  Returns the number of candidates (None
+    with --tuning); their times, 8 KB of them, go to stderr, so that the result line stays short."""
     if getattr(args, "quorum", None) is not None:
         eng.set_quorum(args.quorum)
     if args.tuning:
@@ -252,7 +253,9 @@ def tune_engine(eng, args, trials):
             if v[6] >= 0:
                 eng.set_first_stage(v[6])
         return None
-    return eng.autotune(trials)
+    table = eng.autotune(trials)
+    print("autotune: " + json.dumps(table), file=sys.stderr)
+    return len(table)
 
 
 def sums(stats, keys=("evaluated", "passed", "accepted")):
@@ -608,7 +611,7 @@ def plain_config2(args, local):
         ms += eng.run_timed(s.n)
     prof = eng.profile(reset=True)
     out = {"workload": CFG2, "particles": s.n, "sweeps_per_s": 3 / (ms / 1e3), "trials_per_s": 3 * s.n / (ms / 1e3),
-           "tuning": eng.tuning(), "autotune": tuned,
+           "tuning": eng.tuning(), "autotune_candidates": tuned,
            "k_mc_share": prof["mc_ms"] / ms if ms else None,
            "k_mc_alg_gbs": prof["mc_alg_bytes"] / (prof["mc_ms"] / 1e3) / 1e9 if prof["mc_ms"] else None}
     eng.close()
@@ -775,7 +778,7 @@ def run_ours(args):
             "config": workload_config(len(n_all), n_all),
             "step": {"trials_per_replica": T, "sweeps": total_sweeps_per_step, "replicas_this_rank": len(reps),
                      "l2": "flushed between steps (256 MiB write on the engine stream)"},
-            "tuning": {"chosen": eng.tuning(), "autotune": tune, "da_threshold": args.da_threshold},
+            "tuning": {"chosen": eng.tuning(), "autotune_candidates": tune, "da_threshold": args.da_threshold},
             "roofline": dict(rl[dominant], kernel=dominant) if dominant else None,
             "roofline_other": {k: v for k, v in rl.items() if k != dominant},
             "e2e": e2e, "gpu_launches": int(prof["kernel_launches"]),
