@@ -41,8 +41,7 @@ namespace cg = cooperative_groups;
 #define RUN_HIT 64
 #define RUN_TAB(p) (2 * Win<p>::TAB)  // floats of a warp's window tables
 
-// A block's stencil and probe tables, trials and counters of one batch (one object, so that the
-// other blocks of a cluster can copy it).
+// One trial of a batch: its changes, bonds, stencils and probes, and the terms that need no other particle.
 struct RunTrial {
     int move, skip, nch, nst, st0, np, p0, lists;
     int idx[2], pres_old[2], pres_new[2], to[2], tn[2], fo[2];
@@ -153,6 +152,8 @@ __host__ __device__ constexpr size_t run_stencil_bytes(int pend_max) {
     return (sizeof(PadSt<P>) * (pend_max + RUN_TST) + 15) / 16 * 16;
 }
 
+// A block's probe tables, trials and counters of one batch (one object, so that the other blocks of a
+// cluster can copy it).
 struct __align__(16) RunShared {
     RunTrial T[RUN_BATCH];
     float4 pp[RUN_PROBES];                  // probes: position, type, sign, trial, which change

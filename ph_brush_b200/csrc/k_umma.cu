@@ -244,7 +244,7 @@ __global__ void __launch_bounds__(UM_NT, 1) k_umma_gemm(int M, int N, int K, con
         // each warp moves its 32 TMEM lanes (rows; a warp reaches the 32 of its number mod 4)
         // through shared memory, UM_EC columns at a time (the stages are
         // free once every MMA has completed), so that the epilogue's loads and stores run along
-        // the rows; the two warps of a row group take column blocks in turn
+        // the rows; the four warps of a row group take column blocks in turn
         float* tile = reinterpret_cast<float*>(um_smem) + warp * (32 * (UM_EC + 1));
         if (epi == 0) Cf += (size_t)blockIdx.z * M * N;
         const int wr = warp & 3;
@@ -319,7 +319,7 @@ __global__ void __launch_bounds__(UM_NT, 1) k_umma_gemm(int M, int N, int K, con
 }
 
 // Shared memory of one launch: two stages of A (128 x 64) and B (Np x 64) BF16, at least the
-// epilogue's 32 x 65 float tile per warp.
+// epilogue's 32 x 33 float tile per warp.
 static size_t umma_gemm_smem(int N) {
     const int Np = (N + 15) & ~15;
     const size_t stages = (size_t)2 * (UM_ROWS * UM_KC * 2 + Np * UM_KC * 2);
