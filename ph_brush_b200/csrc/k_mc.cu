@@ -797,6 +797,33 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_mc(DevPtrs d, int mode, int ex
     };
     __syncthreads();
 
+    // z-density sample after every zh_every trials of the run, whatever became of the trial (S.trial was
+    // advanced by its proposal, at least one barrier ago, so every thread sees one value)
+    auto z_sample = [&]() {
+        if (GC || mode != MC_RUN || d.zh_bins <= 0 || S.trial % d.zh_every != 0) return;
+        const int nb = d.zh_bins;
+        for (int k = tid; k < 3 * nb; k += NT) s_zh[k] = 0u;
+        __syncthreads();
+        const float z0 = D.walls ? D.wall_lo : 0.0f;
+        const float inv = (float)nb / (D.walls ? (D.wall_hi - D.wall_lo) : D.L[2]);
+        for (int i = tid; i < D.cap; i += NT) {
+            const int fl = d.flags[D.slot_off + i];
+            if (fl & PHMC_F_GHOST) continue;
+            const float4 pq = d.posq[D.slot_off + i];
+            int cls = -1;
+            if (fl & PHMC_F_TITRATABLE) cls = pq.w != 0.0f ? 0 : -1;
+            else if (fl & PHMC_F_ANION) cls = 1;
+            else if (fl & PHMC_F_CATION) cls = 2;
+            if (cls < 0) continue;
+            const int b = min(max((int)((pq.z - z0) * inv), 0), nb - 1);
+            atomicAdd(&s_zh[cls * nb + b], 1u);
+        }
+        __syncthreads();
+        unsigned long long* h = d.zhist + (size_t)r * 3 * nb;  // this replica's row: one block, no race
+        for (int k = tid; k < 3 * nb; k += NT) h[k] += s_zh[k];
+        if (tid == 0) d.zh_samples[r] += 1;
+        __syncthreads();
+    };
     for (;;) {
         // ---------------- proposal ----------------
         if (tid < 32) {
@@ -1087,6 +1114,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_mc(DevPtrs d, int mode, int ex
                 }
             }
             __syncthreads();
+            z_sample();
             mark(7);
             continue;
         }
@@ -1545,32 +1573,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_mc(DevPtrs d, int mode, int ex
                 __syncthreads();
             }
         }
-        // z-density sample after every zh_every trials of the run (S.trial was advanced by
-        // this trial's proposal before the barriers above, so every thread sees one value)
-        if (!GC && mode == MC_RUN && d.zh_bins > 0 && S.trial % d.zh_every == 0) {
-            const int nb = d.zh_bins;
-            for (int k = tid; k < 3 * nb; k += NT) s_zh[k] = 0u;
-            __syncthreads();
-            const float z0 = D.walls ? D.wall_lo : 0.0f;
-            const float inv = (float)nb / (D.walls ? (D.wall_hi - D.wall_lo) : D.L[2]);
-            for (int i = tid; i < D.cap; i += NT) {
-                const int fl = d.flags[D.slot_off + i];
-                if (fl & PHMC_F_GHOST) continue;
-                const float4 pq = d.posq[D.slot_off + i];
-                int cls = -1;
-                if (fl & PHMC_F_TITRATABLE) cls = pq.w != 0.0f ? 0 : -1;
-                else if (fl & PHMC_F_ANION) cls = 1;
-                else if (fl & PHMC_F_CATION) cls = 2;
-                if (cls < 0) continue;
-                const int b = min(max((int)((pq.z - z0) * inv), 0), nb - 1);
-                atomicAdd(&s_zh[cls * nb + b], 1u);
-            }
-            __syncthreads();
-            unsigned long long* h = d.zhist + (size_t)r * 3 * nb;  // this replica's row: one block, no race
-            for (int k = tid; k < 3 * nb; k += NT) h[k] += s_zh[k];
-            if (tid == 0) d.zh_samples[r] += 1;
-            __syncthreads();
-        }
+        z_sample();
         mark(6);
     }
     if constexpr (GC) {
