@@ -233,7 +233,7 @@ __global__ void k_out_backward(const float* __restrict__ dy, const float* __rest
 // (job l: sum_i dZ_l[i][j]), and (job 3) dw4[j] = sum_i dy_i H3[i][j] with db4 = sum_i dy_i.  A block
 // sums a range of rows, lanes on consecutive column pairs, eight rows at a time as a tree; a job's last
 // block adds the blocks' sums, trees of 32 and FP64 over those.  (A block per column read its column with
-// a stride of a row: 45 us for the four at 16384 x 128, 14 us here.  Error against 64 bits of sums of 16384
+// a stride of a row: 45 us for the four at 16384 x 128, 16 us here.  Error against 64 bits of sums of 16384
 // normal numbers of mean 0.05: 4.2e-5 in 256 strided parts as that kernel had them, 2.7e-5 here, 1.1e-4
 // with the rows and the blocks each in one chain.)
 #define CSUM_NB 128

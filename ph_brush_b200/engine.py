@@ -193,7 +193,7 @@ class Engine:
         return t.asdict()
 
     def autotune(self, trials):
-        """Every candidate timed (z pass: rebuild_us; full-recompute block: recompute_us; pending
+        """Every candidate with its time (z pass: rebuild_us; full-recompute block: recompute_us; pending
         capacity x threads and pair-pass round width: us_per_trial); the engine keeps the best."""
         res = (_abi.Tuning * 64)()
         n = C.c_int()
