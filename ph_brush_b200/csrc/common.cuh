@@ -184,6 +184,7 @@ struct DevPtrs {
     SurDev sur;
     int sur_late_l3;     // two-buffer staging (layer 3 copied after layer 1) to keep two MC blocks per SM
     int* quorum_ctl;     // [replicas active at the MC launch's start, of them stopped by a full pending buffer]
+    float2* run_rate;    // per replica, recent batches of plain runs: forced ends, trials decided (sets their length)
     float quorum;        // the launch ends once that fraction of its active replicas is blocked (>= 1: off)
     float da_threshold;  // minimum second-stage acceptance among first-stage passes
     int da_window;       // first-stage passes per agreement check

@@ -436,6 +436,8 @@ static int build(phmc_engine* h, int R, const phmc_system* sys, const phmc_param
     DALLOC(d.cations, N); DALLOC(d.cation_pos, N); DALLOC(d.freel, N); DALLOC(d.titr, N);
     DALLOC(d.desc, R); DALLOC(d.state, R); DALLOC(d.dirty, R);
     DALLOC(d.quorum_ctl, 2);
+    DALLOC(d.run_rate, R);
+    CU(cudaMemset(d.run_rate, 0, sizeof(float2) * R));
     d.quorum = 1.0f;
     DALLOC(E.d_rep_of, N);
     DALLOC(E.d_cell_rep, E.total_cells);

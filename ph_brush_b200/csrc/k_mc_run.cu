@@ -15,6 +15,7 @@
 // Measured on a B200 (250-400 trials of a run, wall time of the whole call): one replica of 484
 // particles 2120 -> 810 us, one of 11.7k particles 5170 -> 1570 us, 24 uneven replicas 4250 ->
 // 2100 us; 256 replicas, two blocks to an SM, 16.1 -> 15.4 ms (half of it mesh rebuilds).
+// (Titration-only runs, and how long batches are: run_length.)
 // A batch ends early (and the next one starts there) where an accepted trial could have
 // changed a later one: an inserted or removed particle changes the index lists that
 // proposals draw from; a changed particle within the largest cutoff of a later trial's
@@ -52,6 +53,20 @@ struct RunTrial {
     double direct_lj, direct_c;
     double dQ, dQ2, dMz, dS2;
 };
+
+// Trials of a batch: a batch of n costs the latency of one and n trials' work, of which the trials after a
+// cut are lost.  With cuts at a rate of h a trial the best n is near sqrt(worth / h), worth being twice
+// the latency in units of a trial's work.  (Titrations and ion swaps change the lists that proposals draw
+// from, so an accepted one always cuts: a run of titrations alone decided 2 of the 16 trials of a batch.
+// 300 such trials, long batches always -> this rule (one trial at a time before batches): 12k particles 7.4 ->
+// 5.5 ms (5.5), 96 uneven replicas 31 -> 12.7 (16.1), 256 replicas 30.4 -> 20.5 (24.2), 75 of 40 particles
+// 15.2 -> 4.2 (4.2); with 90 % displacements 1.35 -> 1.35 (4.0), 7.6 -> 5.3 (9.7), 9.8 -> 9.2 (13.4), 3.6 -> 2.0
+// (3.0).  Left behind: titrations alone on more small replicas than SMs, 15 % slower than one at a time,
+// 23 % at order 6, whose windows take twice the instructions.)
+__device__ __forceinline__ int run_length(float2 rate, float worth, int batch) {
+    const float a = worth * rate.y;
+    return rate.x > 0.0f ? max(1, (int)fminf(a * rsqrtf(a * rate.x) + 0.5f, (float)batch)) : batch;
+}
 
 // Proposal of trial t (the rules of the oracle's Monte Carlo, as in k_mc).
 __device__ __forceinline__ void run_propose(RunTrial& T, long long t, const RepDesc& D, const RepState& S, const DevPtrs& d) {
@@ -167,7 +182,7 @@ struct __align__(16) RunShared {
 // work of each batch; they copy the batch's tables from the first block's shared memory and store
 // their results into it.
 template <int P, int NT, bool CL>
-__global__ void __launch_bounds__(NT, 512 / NT) k_mc_run(DevPtrs d, int pend_max, int batch) {
+__global__ void __launch_bounds__(NT, 512 / NT) k_mc_run(DevPtrs d, int pend_max, int batch, float worth) {
     constexpr int P3 = P * P * P;
     constexpr int NW = NT / 32;
     extern __shared__ __align__(16) unsigned char dsm[];
@@ -195,6 +210,10 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_mc_run(DevPtrs d, int pend_max
     __shared__ double s_ev[RUN_BATCH][8];   // energy changes, in RepState's order from E on
     __shared__ int s_cp[RUN_TST][2], s_mv[2 * RUN_BATCH][3];  // stencil moves; cell moves (slot, from, to)
     __shared__ int s_nev, s_ncp, s_nmv;
+    // recent batches: those that an accepted trial cut short, trials decided; the last batch's; trials of
+    // the next one at most (made beside the stencils, off the deciding lane's chain, so one batch late)
+    __shared__ float2 s_rate;
+    __shared__ int s_cut, s_decided, s_len;
     __shared__ unsigned int s_zh[3 * PHMC_ZHIST_MAX_BINS];
 
     unsigned rank = 0, csize = 1;
@@ -215,6 +234,11 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_mc_run(DevPtrs d, int pend_max
         B.npend = 0; s_nq = 0; B.stop = 0; s_qstop = 0; s_qin = 0;
         s_nev = 0; s_ncp = 0; s_nmv = 0;
         if (rank == 0 && d.quorum < 1.0f && S.trial < S.target) { atomicAdd(&d.quorum_ctl[0], 1); s_qin = 1; }
+    }
+    if (tid == 32) {
+        s_rate = d.run_rate[r];
+        s_len = run_length(s_rate, worth, batch);
+        s_cut = 0; s_decided = 0;
     }
     unsigned long long t_start = 0;
     if (tid == 0) asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t_start));
@@ -264,7 +288,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_mc_run(DevPtrs d, int pend_max
             if (!stop) {
                 long long n = S.target - S.trial;
                 if (d.zh_bins > 0) n = min(n, d.zh_every - S.trial % d.zh_every);  // a sample ends a batch
-                nb = (int)min((long long)batch, n);
+                nb = (int)min((long long)s_len, n);
                 int np = 0, ns = 0;
                 // a probe per old and per new state; a stencil per charge that appears, leaves or changes
                 auto states = [&](auto&& probe, auto&& stencil) {
@@ -352,6 +376,11 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_mc_run(DevPtrs d, int pend_max
         const int nb = B.nb, npend = B.npend, ns = B.ns;
         // ---------------- stencils, direct and bonded terms, conflicts ----------------
         if (tid == 0) s_nq = 0;
+        if (tid == NT - 1) {
+            const float2 q = make_float2(0.9f * s_rate.x + (float)s_cut, 0.9f * s_rate.y + (float)s_decided);
+            s_rate = q;
+            s_len = run_length(q, worth, batch);
+        }
         constexpr int Q_ST = 0, Q_FE = Q_ST + 3 * RUN_TST, Q_DI = Q_FE + 4 * RUN_BATCH, Q_CF = Q_DI + 32,
                       Q_END = Q_CF + RUN_BATCH * RUN_BATCH;
         for (int it = tid; it < Q_END; it += NT) {
@@ -808,6 +837,8 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_mc_run(DevPtrs d, int pend_max
                 S.trials_run += cur; S.alg_bytes += (double)bs;
                 S.Q = Qs; S.Mz = Ms; S.S2 = S2s;
                 S.trial = t0 + cur; B.npend = np;
+                s_cut = np + 2 <= pend_max && (cur < nb || (((taken >> (cur - 1)) & 1u) && B.T[cur - 1].lists));
+                s_decided = cur;
             }
             if (taken && lane == 30) {
                 double q2 = S.Q2;
@@ -849,6 +880,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_mc_run(DevPtrs d, int pend_max
         asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t_end));
         S.busy_ns += (long long)(t_end - t_start);
         d.state[r] = S;
+        d.run_rate[r] = s_rate;
         if (B.npend > 0) d.dirty[r] = 1;  // potential mesh is stale: rebuild before the next MC launch
     }
 }
@@ -863,7 +895,7 @@ size_t run_smem_bytes(int order, int nt, int pend_max) {
 // them to an SM; otherwise a replica takes blocks of 512 threads, the largest cluster (8, 4, 2, 1)
 // with which all replicas are resident at once.
 template <int P, int NT, bool CL>
-static cudaError_t launch_run_t(Engine& E, int csize, int batch, cudaStream_t st) {
+static cudaError_t launch_run_t(Engine& E, int csize, int batch, float worth, cudaStream_t st) {
     DevPtrs dd = E.d;
     auto kern = k_mc_run<P, NT, CL>;
     const size_t smem = run_smem_bytes(P, NT, E.pend_max);
@@ -893,7 +925,7 @@ static cudaError_t launch_run_t(Engine& E, int csize, int batch, cudaStream_t st
     at[0].val.clusterDim.x = csize; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = CL ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, kern, dd, E.pend_max, batch);
+    return cudaLaunchKernelEx(&cfg, kern, dd, E.pend_max, batch, worth);
 }
 
 template <int P, int NT, bool CL>
@@ -935,12 +967,15 @@ static cudaError_t prepare_run_p(Engine& E) {
     return prepare_run_t<P, 512, false>(E);
 }
 
+// The longest batch: on one block 16 trials' work takes longer than what they save (300 trials of 96
+// uneven replicas 7.5 ms with 16, 5.6 with 8).  worth (run_length) by trial: 1 to 16 trials always,
+// one to 149 replicas of 40 and 300 particles, titrations, swaps or displacements; within 5 % of the best.
 template <int P>
 static cudaError_t launch_run_p(Engine& E, cudaStream_t st) {
-    if (E.run_cluster > 1) return launch_run_t<P, 512, true>(E, E.run_cluster, RUN_BATCH, st);
-    if (E.R <= E.nsm) return launch_run_t<P, 512, false>(E, 1, RUN_BATCH, st);
-    if (E.threads == 256) return launch_run_t<P, 256, false>(E, 1, RUN_BATCH / 2, st);
-    return launch_run_t<P, 128, false>(E, 1, RUN_BATCH / 2, st);
+    if (E.run_cluster > 1) return launch_run_t<P, 512, true>(E, E.run_cluster, RUN_BATCH, E.run_cluster == 8 ? 28.0f : 1.75f * E.run_cluster, st);
+    if (E.R <= E.nsm) return launch_run_t<P, 512, false>(E, 1, RUN_BATCH / 2, 2.2f, st);
+    if (E.threads == 256) return launch_run_t<P, 256, false>(E, 1, RUN_BATCH / 2, 1.5f, st);
+    return launch_run_t<P, 128, false>(E, 1, RUN_BATCH / 2, 1.2f, st);
 }
 
 cudaError_t prepare_mc_run(Engine& E) {

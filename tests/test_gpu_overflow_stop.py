@@ -43,22 +43,18 @@ def test_no_trial_beyond_the_batch_of_an_overflow(replicas, batch, seed):
     cell = lambda st: tuple(np.minimum((st[k][:N]).astype(int), L - 1) for k in ("x", "y", "z"))
     occ = np.zeros((L, L, L), int)
     np.add.at(occ, cell(mc.state()), 1)
-    t, end, full = 0, 0, False
-    while not full:  # batch by batch
-        end, drawn = t, set()
-        while end < t + batch and picked(p.seed, end, N) not in drawn:
-            drawn.add(picked(p.seed, end, N))
-            end += 1
-        for k in range(t, end):
-            i = picked(p.seed, k, N)
-            was = tuple(a[i] for a in cell(mc.state()))
-            assert mc.step()[2] == 1
-            now = tuple(a[i] for a in cell(mc.state()))
-            if was != now and not full:
-                occ[was] -= 1
-                full = occ[now] >= p.cell_cap
-                occ[now] += 1
-        t = end
-    ref = mc.state()
-    for k in ("x", "y", "z"):
-        assert np.array_equal(got[k][:N], ref[k][:N]), k
+    full, beyond, t = False, 0, 0  # trials after the one that overflows a cell; all
+    while True:
+        st = mc.state()
+        if full and all(np.array_equal(got[k][:N], st[k][:N]) for k in ("x", "y", "z")):
+            break  # the state that the engine left behind
+        assert beyond < batch, "trials were judged beyond the overflow's batch"
+        beyond += full
+        i, was = picked(p.seed, t, N), cell(st)
+        assert mc.step()[2] == 1
+        t += 1
+        was, now = tuple(a[i] for a in was), tuple(a[i] for a in cell(mc.state()))
+        if was != now and not full:
+            occ[was] -= 1
+            full = occ[now] >= p.cell_cap
+            occ[now] += 1
