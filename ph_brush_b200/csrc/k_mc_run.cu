@@ -972,7 +972,7 @@ static cudaError_t prepare_run_p(Engine& E) {
 // one to 149 replicas of 40 and 300 particles, titrations, swaps or displacements; within 5 % of the best.
 template <int P>
 static cudaError_t launch_run_p(Engine& E, cudaStream_t st) {
-    if (E.run_cluster > 1) return launch_run_t<P, 512, true>(E, E.run_cluster, RUN_BATCH, E.run_cluster == 8 ? 28.0f : 1.75f * E.run_cluster, st);
+    if (E.run_cluster > 1) return launch_run_t<P, 512, true>(E, E.run_cluster, RUN_BATCH, E.run_cluster == 8 ? 28.0f : 2.5f * E.run_cluster, st);
     if (E.R <= E.nsm) return launch_run_t<P, 512, false>(E, 1, RUN_BATCH / 2, 2.2f, st);
     if (E.threads == 256) return launch_run_t<P, 256, false>(E, 1, RUN_BATCH / 2, 1.5f, st);
     return launch_run_t<P, 128, false>(E, 1, RUN_BATCH / 2, 1.2f, st);
