@@ -211,7 +211,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_mc_run(DevPtrs d, int pend_max
     __shared__ int s_cp[RUN_TST][2], s_mv[2 * RUN_BATCH][3];  // stencil moves; cell moves (slot, from, to)
     __shared__ int s_nev, s_ncp, s_nmv;
     // recent batches: those that an accepted trial cut short, trials decided; the last batch's; trials of
-    // the next one at most (made beside the stencils, off the deciding lane's chain, so one batch late)
+    // the next one at most (made beside the pair terms, off the deciding lane's chain, so one batch late)
     __shared__ float2 s_rate;
     __shared__ int s_cut, s_decided, s_len;
     __shared__ unsigned int s_zh[3 * PHMC_ZHIST_MAX_BINS];
@@ -376,11 +376,6 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_mc_run(DevPtrs d, int pend_max
         const int nb = B.nb, npend = B.npend, ns = B.ns;
         // ---------------- stencils, direct and bonded terms, conflicts ----------------
         if (tid == 0) s_nq = 0;
-        if (tid == NT - 1) {
-            const float2 q = make_float2(0.9f * s_rate.x + (float)s_cut, 0.9f * s_rate.y + (float)s_decided);
-            s_rate = q;
-            s_len = run_length(q, worth, batch);
-        }
         constexpr int Q_ST = 0, Q_FE = Q_ST + 3 * RUN_TST, Q_DI = Q_FE + 4 * RUN_BATCH, Q_CF = Q_DI + 32,
                       Q_END = Q_CF + RUN_BATCH * RUN_BATCH;
         for (int it = tid; it < Q_END; it += NT) {
@@ -605,6 +600,11 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_mc_run(DevPtrs d, int pend_max
             alj = warp_sum(alj);
             ac = warp_sum(ac);
             if (lane == 0) { r_plj[p] = alj; r_pc[p] = ac; r_pn[p] = total; }
+        }
+        if (rank == 0 && tid == NT - 1) {
+            const float2 q = make_float2(0.9f * s_rate.x + (float)s_cut, 0.9f * s_rate.y + (float)s_decided);
+            s_rate = q;
+            s_len = run_length(q, worth, batch);
         }
         if (d.phase_clk) { __syncthreads(); mark(4); }
         // ---------------- mesh terms ----------------
